@@ -220,9 +220,13 @@ int qgb_project(int dtype, const void* beta, const void* C, void* projT, int nk,
  * complex128 [nk][nx][ny] for both dtypes (FP32 inputs: FP32 partial sums,
  * added in FP64).  Replaces Wavefunction.dot / ^ for one spin and no spinors
  * (qimpy/dft/electrons/_wavefunction_dot.py:18-107).  Workspace of
- * qgb_dot_workspace_bytes (split-K partials, fixed summation order).
+ * qgb_dot_workspace_bytes (split-K partials, fixed summation order, so repeated
+ * calls give equal bits).  With qgb_dot_fast_workspace_bytes (>= that) the larger
+ * FP64 products run on the tensor cores as integer slices, to FP64 accuracy;
+ * this holds for qgb_project (nx = P, ny = nb) and qgb_dot_real (nk = 1) too.
  */
 size_t qgb_dot_workspace_bytes(int dtype, int nk, int nx, int ny, int n_tot);
+size_t qgb_dot_fast_workspace_bytes(int dtype, int nk, int nx, int ny, int n_tot);
 int qgb_dot(int dtype, const void* X, int nx, const void* Y, int ny, int nk, int n_tot, void* out,
             void* workspace, size_t workspace_bytes, void* stream);
 /*
@@ -262,9 +266,17 @@ int qgb_dot_real(int dtype, const void* X, int nx, const void* Y, int ny, int n_
  * QGB_ACCUMULATE) for C [nk][n_in][n_tot], M [nk][n_in][n_out] and out
  * [nk][n_out][n_tot], all of `dtype`; out must not alias C.  Replaces
  * Wavefunction.matmul / @ (qimpy/dft/electrons/_wavefunction_dot.py:137-191).
+ *
+ * qgb_matmul_ws is the same with a workspace of qgb_matmul_workspace_bytes (0:
+ * none needed), with which the larger FP64 rotations run on the tensor cores
+ * (integer slices, FP64 accuracy); a smaller or NULL workspace, and qgb_matmul,
+ * run on the FP64 pipe.
  */
 int qgb_matmul(int dtype, const void* C, int n_in, int nk, int n_tot, const void* M, int n_out, void* out,
                unsigned flags, void* stream);
+size_t qgb_matmul_workspace_bytes(int dtype, int nk, int n_in, int n_out, int n_tot);
+int qgb_matmul_ws(int dtype, const void* C, int n_in, int nk, int n_tot, const void* M, int n_out, void* out,
+                  unsigned flags, void* workspace, size_t workspace_bytes, void* stream);
 
 /*
  * out[k][b][g] += sum_p beta[k][p][g] (D_all projT[k][b])[p]  (replaces

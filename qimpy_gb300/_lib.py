@@ -112,6 +112,10 @@ _SIGS = {
                                        ct.POINTER(QgbProjectorShell), ct.c_double, ct.c_void_p, ct.c_void_p]),
     "qgb_matmul": (ct.c_int, [ct.c_int, ct.c_void_p, ct.c_int, ct.c_int, ct.c_int, ct.c_void_p, ct.c_int,
                               ct.c_void_p, ct.c_uint, ct.c_void_p]),
+    "qgb_dot_fast_workspace_bytes": (ct.c_size_t, [ct.c_int, ct.c_int, ct.c_int, ct.c_int, ct.c_int]),
+    "qgb_matmul_workspace_bytes": (ct.c_size_t, [ct.c_int, ct.c_int, ct.c_int, ct.c_int, ct.c_int]),
+    "qgb_matmul_ws": (ct.c_int, [ct.c_int, ct.c_void_p, ct.c_int, ct.c_int, ct.c_int, ct.c_void_p, ct.c_int,
+                                 ct.c_void_p, ct.c_uint, ct.c_void_p, ct.c_size_t, ct.c_void_p]),
     "qgb_apply_nonlocal": (ct.c_int, [ct.c_int, ct.c_void_p, ct.c_void_p, ct.c_int, ct.c_int, ct.c_void_p,
                                       ct.c_void_p, ct.c_int, ct.c_int, ct.c_int, ct.c_void_p, ct.c_void_p]),
     "qgb_hamiltonian": (ct.c_int, [ct.POINTER(QgbSphere), ct.c_int, ct.c_void_p, ct.c_void_p, ct.c_int,

@@ -9,8 +9,9 @@
 //   rotate  out[j][g] (+)= sum_i W(i, j) X[i][g]         (short i, long g)
 //   dapply  Dp[b][a pa + r] = sum_c D[a][r][c] proj[b][a pa + c]
 // Arrays are batched over k-points with explicit strides.  GB300's FP64 rate
-// (about 1 TFLOP/s) bounds the FP64 products, so they are register-tiled DFMA
-// loops with shared-memory staging; the FP32 forms use the same tiling.
+// (about 1 TFLOP/s) bounds the FP64 forms here, register-tiled multiply-add
+// loops with shared-memory staging; larger FP64 products given a workspace go
+// to the tensor cores instead (ozaki.cu).  The FP32 forms use the same tiling.
 // Every product is deterministic: split-K partial tiles are summed by a
 // second kernel in a fixed order (no atomics), so repeated calls, and calls
 // from different host threads, give identical bits.
@@ -315,10 +316,17 @@ __global__ void k_dapply(const cplx_t<T>* __restrict__ proj, const cplx_t<T>* __
 
 using namespace bg;
 
-// Workspace (bytes) of a Gram product: the split-K partial tiles.
-size_t gram_workspace_bytes(int dtype, int nk, int M, int N, int K) {
+size_t gram_workspace_bytes(int dtype, int nk, int M, int N, int K, bool sliced) {
   if (nk < 1 || M < 1 || N < 1 || K < 1) return 0;
-  return gram_plan(nk, M, N, K, elem_bytes(dtype)).partial_bytes;
+  const size_t partial = gram_plan(nk, M, N, K, elem_bytes(dtype)).partial_bytes;
+  if (!sliced || dtype != QGB_F64 || !oz_gram_use(nk, M, N, K)) return partial;
+  return std::max(partial, std::max(oz_gram_workspace_bytes(nk, M, N, K, false),
+                                    oz_gram_workspace_bytes(nk, M, N, K, true)));
+}
+
+size_t rotate_workspace_bytes(int dtype, int nk, int Kin, int Nout, int G) {
+  if (nk < 1 || Kin < 1 || Nout < 1 || G < 1 || dtype != QGB_F64 || !oz_rotate_use(nk, Kin, Nout, G)) return 0;
+  return oz_rotate_workspace_bytes(nk, Kin, Nout, G);
 }
 
 template <typename T, typename OutT>
@@ -342,6 +350,9 @@ int gram(int dtype, int out_dtype, const void* A, long long a_batch, int lda, co
   if (out_dtype != QGB_F64 && out_dtype != QGB_F32) return fail(QGB_ERR_INVALID, "unknown out dtype %d", out_dtype);
   if (dtype == QGB_F64 && out_dtype == QGB_F32) return fail(QGB_ERR_UNSUPPORTED, "FP64 gram to FP32 output");
   if (K == 0) return fail(QGB_ERR_INVALID, "gram over an empty basis");
+  if (dtype == QGB_F64 && ws && oz_gram_use(nk, M, N, K) &&
+      ws_bytes >= oz_gram_workspace_bytes(nk, M, N, K, real_out))
+    return oz_gram(A, a_batch, lda, B, b_batch, ldb, nk, M, N, K, out, out_batch, oi, oj, ws, st, weight, real_out);
   const GramPlan p = gram_plan(nk, M, N, K, elem_bytes(dtype));
   if (p.splits > 1 && (!ws || ws_bytes < p.partial_bytes))
     return fail(QGB_ERR_WORKSPACE, "gram workspace %zu B < %zu B", ws_bytes, p.partial_bytes);
@@ -377,10 +388,13 @@ int gram(int dtype, int out_dtype, const void* A, long long a_batch, int lda, co
 // out[k][j][g] (+)= sum_i W(i, j) X[k][i][g] with W(i, j) = W[k*w_batch + i*wi + j*wj].
 int rotate(int dtype, const void* X, long long x_batch, int ldx, const void* W, long long w_batch, int wi, int wj,
            int nk, int Kin, int Nout, int G, void* out, long long out_batch, int ldo, bool accumulate,
-           cudaStream_t st) {
+           cudaStream_t st, void* ws, size_t ws_bytes) {
   if (nk < 0 || Kin < 0 || Nout < 0 || G < 0) return fail(QGB_ERR_INVALID, "negative rotate extent");
   if (nk == 0 || Nout == 0 || G == 0) return QGB_OK;
   if (!out || (Kin > 0 && (!X || !W))) return fail(QGB_ERR_INVALID, "NULL pointer in rotate");
+  if (dtype == QGB_F64 && Kin > 0 && ws && oz_rotate_use(nk, Kin, Nout, G) &&
+      ws_bytes >= oz_rotate_workspace_bytes(nk, Kin, Nout, G))
+    return oz_rotate(X, x_batch, ldx, W, w_batch, wi, wj, nk, Kin, Nout, G, out, out_batch, ldo, accumulate, ws, st);
   RotArgs r{X, W, out, x_batch, w_batch, out_batch, ldx, ldo, wi, wj, Kin, Nout, G, accumulate ? 1 : 0};
   if (dtype == QGB_F64) {
     constexpr int TJ = 4;

@@ -1,4 +1,5 @@
 // extern "C" entry points of libqimpy_gb300 (declared in include/qimpy_gb300.h).
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <map>
@@ -51,11 +52,12 @@ int apply_potential(const qgb_sphere* s, int dtype, const void* C, void* out, in
                     void* ws, size_t ws_bytes, cudaStream_t st,
                     cudaEvent_t gather_after = nullptr);
 int apply_ke(const qgb_sphere* s, int dtype, const void* C, void* out, int nb, cudaStream_t st);
-size_t project_workspace_bytes(int dtype, int nk, int P, int nb, int n_tot);
+size_t project_workspace_bytes(int dtype, int nk, int P, int nb, int n_tot, bool sliced = true);
 int project(int dtype, const void* beta, const void* C, void* projT, int nk, int P, int nb, int n_tot, void* ws,
             size_t ws_bytes, cudaStream_t st);
 int apply_nonlocal(int dtype, const void* beta, const void* D, int n_atoms, int pa, const void* projT,
-                   void* out, int nk, int nb, int n_tot, void* work, cudaStream_t st);
+                   void* out, int nk, int nb, int n_tot, void* work, cudaStream_t st, void* ws = nullptr,
+                   size_t ws_bytes = 0);
 #ifdef QGB_DEBUG_CHECKS
 int debug_violation(unsigned long long* out4);
 #endif
@@ -129,12 +131,15 @@ size_t qgb_potential_workspace_bytes(const qgb_sphere* s, int nb, int dtype) {
 
 static inline size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
-// Workspace of qgb_hamiltonian: [D proj (nk nb P complex) | <beta|psi> split-K
-// partials | slab planes], each part 256-byte aligned.
-static size_t ham_nonlocal_bytes(const qgb_sphere& s, int nb, int P, int dtype) {
+// Workspace of qgb_hamiltonian: [D proj (nk nb P complex) | workspace of <beta|psi>
+// and then of the back-projection | slab planes], each part 256-byte aligned.
+// Without `sliced`, what the multiply-add kernels need alone: a caller's
+// workspace that holds no more than that is still taken.
+static size_t ham_nonlocal_bytes(const qgb_sphere& s, int nb, int P, int dtype, bool sliced = true) {
   if (P == 0 || nb == 0) return 0;
-  return align256(static_cast<size_t>(s.nk) * nb * P * elem_bytes(dtype)) +
-         align256(project_workspace_bytes(dtype, s.nk, P, nb, s.n_tot));
+  size_t prod = project_workspace_bytes(dtype, s.nk, P, nb, s.n_tot, sliced);
+  if (sliced) prod = std::max(prod, rotate_workspace_bytes(dtype, s.nk, P, nb, s.n_tot));
+  return align256(static_cast<size_t>(s.nk) * nb * P * elem_bytes(dtype)) + align256(prod);
 }
 
 size_t qgb_hamiltonian_workspace_bytes(const qgb_sphere* s, int nb, int P, int dtype) {
@@ -166,7 +171,7 @@ int qgb_apply_potential(const qgb_sphere* s, int dtype, const void* C, void* out
 
 size_t qgb_project_workspace_bytes(int dtype, int nk, int P, int nb, int n_tot) {
   if (dtype != QGB_F64 && dtype != QGB_F32) return 0;
-  return project_workspace_bytes(dtype, nk, P, nb, n_tot);
+  return project_workspace_bytes(dtype, nk, P, nb, n_tot, false);
 }
 
 int qgb_project(int dtype, const void* beta, const void* C, void* projT, int nk, int P, int nb, int n_tot,
@@ -177,6 +182,11 @@ int qgb_project(int dtype, const void* beta, const void* C, void* projT, int nk,
 }
 
 size_t qgb_dot_workspace_bytes(int dtype, int nk, int nx, int ny, int n_tot) {
+  if (dtype != QGB_F64 && dtype != QGB_F32) return 0;
+  return gram_workspace_bytes(dtype, nk, nx, ny, n_tot, false);
+}
+
+size_t qgb_dot_fast_workspace_bytes(int dtype, int nk, int nx, int ny, int n_tot) {
   if (dtype != QGB_F64 && dtype != QGB_F32) return 0;
   return gram_workspace_bytes(dtype, nk, nx, ny, n_tot);
 }
@@ -221,8 +231,12 @@ int qgb_dot_real(int dtype, const void* X, int nx, const void* Y, int ny, int n_
               static_cast<cudaStream_t>(stream), weight, true);
 }
 
-int qgb_matmul(int dtype, const void* C, int n_in, int nk, int n_tot, const void* M, int n_out, void* out,
-               unsigned flags, void* stream) {
+size_t qgb_matmul_workspace_bytes(int dtype, int nk, int n_in, int n_out, int n_tot) {
+  return rotate_workspace_bytes(dtype, nk, n_in, n_out, n_tot);
+}
+
+int qgb_matmul_ws(int dtype, const void* C, int n_in, int nk, int n_tot, const void* M, int n_out, void* out,
+                  unsigned flags, void* workspace, size_t workspace_bytes, void* stream) {
   if (dtype != QGB_F64 && dtype != QGB_F32) return fail(QGB_ERR_INVALID, "unknown dtype %d", dtype);
   if (nk < 0 || n_in < 0 || n_out < 0 || n_tot < 1) return fail(QGB_ERR_INVALID, "bad matmul sizes");
   if (flags & ~QGB_ACCUMULATE) return fail(QGB_ERR_INVALID, "unknown matmul flags 0x%x", flags);
@@ -230,7 +244,12 @@ int qgb_matmul(int dtype, const void* C, int n_in, int nk, int n_tot, const void
   // out[k][j][g] = sum_i M[k][i][j] C[k][i][g]: W(i, j) = M[i*n_out + j].
   return rotate(dtype, C, static_cast<long long>(n_in) * n_tot, n_tot, M, static_cast<long long>(n_in) * n_out,
                 n_out, 1, nk, n_in, n_out, n_tot, out, static_cast<long long>(n_out) * n_tot, n_tot,
-                (flags & QGB_ACCUMULATE) != 0, static_cast<cudaStream_t>(stream));
+                (flags & QGB_ACCUMULATE) != 0, static_cast<cudaStream_t>(stream), workspace, workspace_bytes);
+}
+
+int qgb_matmul(int dtype, const void* C, int n_in, int nk, int n_tot, const void* M, int n_out, void* out,
+               unsigned flags, void* stream) {
+  return qgb_matmul_ws(dtype, C, n_in, nk, n_tot, M, n_out, out, flags, nullptr, 0, stream);
 }
 
 int qgb_apply_nonlocal(int dtype, const void* beta, const void* D, int n_atoms, int pa, const void* projT,
@@ -248,7 +267,8 @@ int qgb_hamiltonian(const qgb_sphere* s, int dtype, const void* C, void* HC, int
   if (C == HC) return fail(QGB_ERR_INVALID, "C and HC must not alias");
   if (n_atoms < 0 || pa < 0 || nb < 0) return fail(QGB_ERR_INVALID, "bad nonlocal sizes");
   const int P = n_atoms * pa;
-  const size_t nl = ham_nonlocal_bytes(*s, nb, P, dtype);
+  size_t nl = ham_nonlocal_bytes(*s, nb, P, dtype);
+  if (workspace_bytes < nl + plane_bytes_per_band(*s, dtype)) nl = ham_nonlocal_bytes(*s, nb, P, dtype, false);
   if (workspace_bytes < nl) return fail(QGB_ERR_WORKSPACE, "workspace too small for nonlocal term");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   char* ws = static_cast<char*>(workspace);
@@ -259,7 +279,7 @@ int qgb_hamiltonian(const qgb_sphere* s, int dtype, const void* C, void* HC, int
     const size_t dp = align256(static_cast<size_t>(s->nk) * nb * P * elem_bytes(dtype));
     rc = project(dtype, beta, C, projT, s->nk, P, nb, s->n_tot, ws + dp, nl - dp, st);
     if (rc) return rc;
-    rc = apply_nonlocal(dtype, beta, D, n_atoms, pa, projT, HC, s->nk, nb, s->n_tot, ws, st);
+    rc = apply_nonlocal(dtype, beta, D, n_atoms, pa, projT, HC, s->nk, nb, s->n_tot, ws, st, ws + dp, nl - dp);
     if (rc) return rc;
   }
   return QGB_OK;

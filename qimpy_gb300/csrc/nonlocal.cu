@@ -12,8 +12,8 @@
 
 namespace qgb {
 
-size_t project_workspace_bytes(int dtype, int nk, int P, int nb, int n_tot) {
-  return gram_workspace_bytes(dtype, nk, P, nb, n_tot);
+size_t project_workspace_bytes(int dtype, int nk, int P, int nb, int n_tot, bool sliced) {
+  return gram_workspace_bytes(dtype, nk, P, nb, n_tot, sliced);
 }
 
 int project(int dtype, const void* beta, const void* C, void* projT, int nk, int P, int nb, int n_tot, void* ws,
@@ -27,7 +27,7 @@ int project(int dtype, const void* beta, const void* C, void* projT, int nk, int
 }
 
 int apply_nonlocal(int dtype, const void* beta, const void* D, int n_atoms, int pa, const void* projT, void* out,
-                   int nk, int nb, int n_tot, void* work, cudaStream_t st) {
+                   int nk, int nb, int n_tot, void* work, cudaStream_t st, void* ws, size_t ws_bytes) {
   const int P = n_atoms * pa;
   if (nk < 0 || n_atoms < 0 || pa < 0 || nb < 0 || n_tot < 1)
     return fail(QGB_ERR_INVALID, "bad apply_nonlocal sizes");
@@ -37,7 +37,7 @@ int apply_nonlocal(int dtype, const void* beta, const void* D, int n_atoms, int 
   if (rc) return rc;
   // out[k][b][g] += sum_p beta[k][p][g] Dp[k][b][p]: i = p, j = b, W(p, b) = Dp[b*P + p].
   return rotate(dtype, beta, static_cast<long long>(P) * n_tot, n_tot, work, static_cast<long long>(nb) * P, 1, P,
-                nk, P, nb, n_tot, out, static_cast<long long>(nb) * n_tot, n_tot, true, st);
+                nk, P, nb, n_tot, out, static_cast<long long>(nb) * n_tot, n_tot, true, st, ws, ws_bytes);
 }
 
 }  // namespace qgb

@@ -143,18 +143,22 @@ int check_map(const qgb_real_map* m, const qgb_sphere* full) {
   return QGB_OK;
 }
 
-// Workspace: packed rows Z, their transform W, D proj, Gram partials, slab planes.
+// Workspace: packed rows Z, their transform W, D proj, workspace of the two band
+// products (without `sliced`, of their multiply-add forms), slab planes.
 struct RealLayout {
   size_t z, w, dp, part, planes, total;
 };
-static RealLayout real_layout(const qgb_sphere& full, const qgb_real_map& m, int nb, int P, int dtype) {
+static RealLayout real_layout(const qgb_sphere& full, const qgb_real_map& m, int nb, int P, int dtype,
+                              bool sliced = true) {
   RealLayout L;
   const int nz = (nb + 1) / 2;
   const size_t eb = elem_bytes(dtype);
   L.z = align256(static_cast<size_t>(nz) * m.n_tot_full * eb);
   L.w = L.z;
   L.dp = P > 0 ? align256(static_cast<size_t>(nb) * P * eb) : 0;
-  L.part = P > 0 ? align256(gram_workspace_bytes(dtype, 1, P, nb, m.n_tot_half)) : 0;
+  L.part = P > 0 ? align256(std::max(gram_workspace_bytes(dtype, 1, P, nb, m.n_tot_half, sliced),
+                                    sliced ? rotate_workspace_bytes(dtype, 1, P, nb, m.n_tot_half) : 0))
+                 : 0;
   L.planes = plane_bytes_per_band(full, dtype) * static_cast<size_t>(std::max(nz, 1));
   L.total = L.z + L.w + L.dp + L.part + L.planes;
   return L;
@@ -242,7 +246,8 @@ extern "C" int qgb_hamiltonian_real(const qgb_sphere* full, const qgb_real_map* 
   if (C == HC) return fail(QGB_ERR_INVALID, "C and HC must not alias");
   const int P = n_atoms * pa;
   if (P > 0 && (!beta || !D || !projT)) return fail(QGB_ERR_INVALID, "NULL projector argument with P > 0");
-  const RealLayout L = real_layout(*full, *m, nb, P, dtype);
+  RealLayout L = real_layout(*full, *m, nb, P, dtype);
+  if (workspace_bytes < L.total) L = real_layout(*full, *m, nb, P, dtype, false);
   if (!workspace || workspace_bytes < L.total)
     return fail(QGB_ERR_WORKSPACE, "workspace %zu B < %zu B", workspace_bytes, L.total);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -265,7 +270,7 @@ extern "C" int qgb_hamiltonian_real(const qgb_sphere* full, const qgb_real_map* 
     return rc;
   if ((rc = dapply(dtype, projT, D, n_atoms, pa, nb, 1, Dp, st))) return rc;
   return rotate(dtype, beta, static_cast<long long>(P) * n, n, Dp, static_cast<long long>(nb) * P, 1, P, 1, P, nb, n,
-                HC, static_cast<long long>(nb) * n, n, true, st);
+                HC, static_cast<long long>(nb) * n, n, true, st, part, L.part);
 }
 
 extern "C" int qgb_symmetrize_real(int dtype, const qgb_real_map* m, void* X, int nb, void* stream) {

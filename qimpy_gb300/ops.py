@@ -101,7 +101,7 @@ def project(beta: torch.Tensor, C: torch.Tensor, projT: torch.Tensor | None = No
     beta, C = _plain(beta), _plain(C)
     projT = torch.empty((nk, nb, P), dtype=C.dtype, device=C.device) if projT is None else projT
     lib = _lib.lib()
-    ws = workspace(lib.qgb_project_workspace_bytes(_qdtype(C), nk, P, nb, n_tot), C.device)
+    ws = workspace(lib.qgb_dot_fast_workspace_bytes(_qdtype(C), nk, P, nb, n_tot), C.device)
     _lib.check(lib.qgb_project(_qdtype(C), beta.data_ptr(), C.data_ptr(), projT.data_ptr(), nk, P, nb, n_tot,
                                ws.data_ptr(), ws.numel(), _stream()), "project")
     return projT
@@ -150,7 +150,7 @@ def dot(X: torch.Tensor, Y: torch.Tensor, out: torch.Tensor | None = None, tc: b
         _lib.check(lib.qgb_dot_tc(X.data_ptr(), nx, Y.data_ptr(), ny, nk, n_tot, out.data_ptr(), ws.data_ptr(),
                                   ws.numel(), device_error_word(X.device).data_ptr(), _stream()), "dot_tc")
         return out
-    ws = workspace(lib.qgb_dot_workspace_bytes(qd, nk, nx, ny, n_tot), X.device)
+    ws = workspace(lib.qgb_dot_fast_workspace_bytes(qd, nk, nx, ny, n_tot), X.device)
     _lib.check(lib.qgb_dot(qd, X.data_ptr(), nx, Y.data_ptr(), ny, nk, n_tot, out.data_ptr(), ws.data_ptr(),
                            ws.numel(), _stream()), "dot")
     return out
@@ -190,8 +190,10 @@ def matmul(C: torch.Tensor, M: torch.Tensor, out: torch.Tensor | None = None, ac
                                      ws.data_ptr(), ws.numel(), device_error_word(C.device).data_ptr(), _stream()),
                    "matmul_tc")
         return out
-    _lib.check(_lib.lib().qgb_matmul(_qdtype(C), C.data_ptr(), n_in, nk, n_tot, Mc.data_ptr(), n_out, out.data_ptr(),
-                                     flags, _stream()), "matmul")
+    lib, qd = _lib.lib(), _qdtype(C)
+    ws = workspace(lib.qgb_matmul_workspace_bytes(qd, nk, n_in, n_out, n_tot), C.device)
+    _lib.check(lib.qgb_matmul_ws(qd, C.data_ptr(), n_in, nk, n_tot, Mc.data_ptr(), n_out, out.data_ptr(), flags,
+                                 ws.data_ptr(), ws.numel(), _stream()), "matmul")
     return out
 
 
@@ -478,7 +480,7 @@ def dot_real(X: torch.Tensor, Y: torch.Tensor, weight: torch.Tensor, out: torch.
     elif out.dtype != torch.complex128 or tuple(out.shape) != (1, nx, ny) or not out.is_contiguous():
         raise ValueError("out must be a contiguous complex128 (1, nx, ny) tensor")
     lib = _lib.lib()
-    ws = workspace(lib.qgb_dot_workspace_bytes(_qdtype(X), 1, nx, ny, n_tot), X.device)
+    ws = workspace(lib.qgb_dot_fast_workspace_bytes(_qdtype(X), 1, nx, ny, n_tot), X.device)
     _lib.check(lib.qgb_dot_real(_qdtype(X), X.data_ptr(), nx, Y.data_ptr(), ny, n_tot, _weight_ptr(weight, n_tot),
                                 out.data_ptr(), ws.data_ptr(), ws.numel(), _stream()), "dot_real")
     return out
