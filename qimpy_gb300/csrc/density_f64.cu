@@ -1,0 +1,9 @@
+// Density kernel, FP64.
+#include "density_kernels.cuh"
+
+namespace qgb {
+
+template int launch_density_chunk<double>(const qgb_sphere&, const LocalParams&, const void*, void*, const double*,
+                                    double*, cudaStream_t);
+
+}  // namespace qgb

@@ -21,6 +21,7 @@
 // shared-memory load or store.
 #pragma once
 
+#include "block_fixed.cuh"
 #include "codelets.cuh"
 #include "qgb_common.cuh"
 
@@ -34,7 +35,8 @@ template <typename T> __device__ __forceinline__ cplx_t<T>* smem_c() {
 
 // One codelet applied in place to smem[off + j * stride], j < R, with an
 // optional twiddle multiply by smem[tw + j * tw_stride] (tw < 0: none) on the
-// outputs; the table holds exp(+i...), conjugated when SIGN < 0.
+// outputs; the table holds exp(+i...) (pack_twiddle's form), conjugated when
+// SIGN < 0.
 template <typename T, int S, int R>
 __device__ __forceinline__ void codelet_inplace(int off, int stride, int tw, int tw_stride, int lim,
                                                 int tw_lim) {
@@ -47,21 +49,17 @@ __device__ __forceinline__ void codelet_inplace(int off, int stride, int tw, int
     re[j] = v.x;
     im[j] = v.y;
   }
-  Codelet<R, S>::run(re, im);
+  Block<T, R> x;
+  x.load(re, im);
+  x.template run<S>();
   if (tw >= 0) {
 #pragma unroll
     for (int j = 1; j < R; ++j) {
       if (!QGB_OK_IDX(tw + j * tw_stride, tw_lim, 40 + R)) return;
-      const cplx_t<T> w = sm[tw + j * tw_stride];
-      const T wy = (S > 0) ? w.y : -w.y;
-      const T xr = re[j] * w.x - im[j] * wy;
-      const T xi = re[j] * wy + im[j] * w.x;
-      re[j] = xr;
-      im[j] = xi;
+      x.template twiddle<S>(j, sm[tw + j * tw_stride]);
     }
   }
-#pragma unroll
-  for (int j = 0; j < R; ++j) sm[off + j * stride] = mk<T>(re[j], im[j]);
+  x.store([&](int j, auto value) { sm[off + j * stride] = value(); });
 }
 
 // Geometry of one pass: item `it` in [0, nbatch * nsub) is (batch = it % nbatch,
@@ -107,34 +105,48 @@ __device__ __forceinline__ void run_pass(int R, const Pass ps) {
   }
 }
 
-// Inverse transform (natural -> permuted) of nbatch pencils starting at shared
-// offset `base`, element stride es; twiddles at shared offset W; `lim` bounds
-// the data region.  Ends with __syncthreads().
-template <typename T>
-__device__ __forceinline__ void fft_inverse(int base, const int* bmap, int nbatch, int bstride, int es,
-                                            int L1, int L2, int W, int lim) {
-  if (L2 > 1) {
-    run_pass<T, +1>(L2, Pass{bmap, base, nbatch, bstride, L1, es, L1 * es, W, L2, 1, lim, W + L1 * L2});
-    __syncthreads();
-  }
-  if (L1 > 1) {
-    run_pass<T, +1>(L1, Pass{bmap, base, nbatch, bstride, L2, L1 * es, es, -1, 0, 0, lim, 0});
-    __syncthreads();
-  }
-}
-
-// Forward transform (permuted -> natural) of nbatch pencils.  Ends with __syncthreads().
-template <typename T>
-__device__ __forceinline__ void fft_forward(int base, const int* bmap, int nbatch, int bstride, int es,
-                                            int L1, int L2, int W, int lim) {
-  if (L1 > 1) {
-    run_pass<T, -1>(L1, Pass{bmap, base, nbatch, bstride, L2, L1 * es, es, (L2 > 1) ? W : -1, 1, L2, lim,
-                             W + L1 * L2});
-    __syncthreads();
-  }
-  if (L2 > 1) {
-    run_pass<T, -1>(L2, Pass{bmap, base, nbatch, bstride, L1, es, L1 * es, -1, 0, 0, lim, 0});
-    __syncthreads();
+// One axis of nbatch pencils starting at shared offset `base`, element stride
+// es: inverse (S > 0, natural -> permuted) or forward (S < 0, permuted ->
+// natural); twiddles at shared offset W; `lim` bounds the data region.  Ends
+// with __syncthreads().  The FP64 form runs both passes through one copy of the
+// pass code (14 long codelets); in FP32 a copy each is 9% faster.
+template <typename T, int S>
+__device__ __forceinline__ void fft_axis(int base, const int* bmap, int nbatch, int bstride, int es, int L1, int L2,
+                                         int W, int lim) {
+  if constexpr (sizeof(T) == 8) {
+    const bool single = L1 == 1 || L2 == 1;
+#pragma unroll 1
+    for (int i = single ? 1 : 0; i < 2; ++i) {
+      const bool strided = !single && (i == 0) == (S > 0);  // DFT_L2 over x[n1 + L1 n2]; else DFT_L1 over blocks
+      const bool tw = !single && i == 0;
+      Pass ps{bmap, base, nbatch, bstride, strided ? L1 : L2, strided ? es : L1 * es, strided ? L1 * es : es,
+              tw ? W : -1, S > 0 ? L2 : 1, S > 0 ? 1 : L2, lim, W + L1 * L2};
+      if (single) {
+        ps.nsub = 1;
+        ps.estride = es;
+      }
+      run_pass<T, S>(single ? L1 * L2 : strided ? L2 : L1, ps);
+      __syncthreads();
+    }
+  } else if constexpr (S > 0) {
+    if (L2 > 1) {
+      run_pass<T, +1>(L2, Pass{bmap, base, nbatch, bstride, L1, es, L1 * es, W, L2, 1, lim, W + L1 * L2});
+      __syncthreads();
+    }
+    if (L1 > 1) {
+      run_pass<T, +1>(L1, Pass{bmap, base, nbatch, bstride, L2, L1 * es, es, -1, 0, 0, lim, 0});
+      __syncthreads();
+    }
+  } else {
+    if (L1 > 1) {
+      run_pass<T, -1>(L1, Pass{bmap, base, nbatch, bstride, L2, L1 * es, es, (L2 > 1) ? W : -1, 1, L2, lim,
+                               W + L1 * L2});
+      __syncthreads();
+    }
+    if (L2 > 1) {
+      run_pass<T, -1>(L2, Pass{bmap, base, nbatch, bstride, L1, es, L1 * es, -1, 0, 0, lim, 0});
+      __syncthreads();
+    }
   }
 }
 

@@ -1,0 +1,714 @@
+// Device code and launches of the local-potential kernels (local_potential.cu
+// describes them).  Each precision and form is compiled in a translation unit
+// of its own: local_f32.cu, local_f64.cu, batched_f32.cu, batched_f64.cu and the
+// two density ones.
+#pragma once
+
+#include <algorithm>
+#include <cmath>
+
+#include "fft_steps.cuh"
+
+namespace qgb {
+
+static constexpr int kThreads = 256;
+
+struct LocalParams {
+  int nb_total;  // bands in C / out (stride of the band axis)
+  int b0;        // first band of this chunk
+  int nb;        // bands in this chunk
+  unsigned flags;
+};
+
+template <typename T>
+__device__ __forceinline__ void load_twiddles(int dst, const cplx_t<T>* src, int count) {
+  cplx_t<T>* sm = smem_c<T>();
+  for (int i = threadIdx.x; i < count; i += blockDim.x) sm[dst + i] = pack_twiddle(src[i]);
+}
+
+// Plane workspace index of (k, band-in-chunk, slab).
+__device__ __forceinline__ size_t plane_index(const qgb_sphere& s, int k, int b, int nb, int slab) {
+  return (static_cast<size_t>(k) * nb + b) * s.max_slabs + slab;
+}
+
+__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst))),
+               "l"(gsrc)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// One complex element global -> shared without a register round trip (8 B
+// for FP32, 16 B for FP64): many copies stay in flight per thread.
+template <typename T>
+__device__ __forceinline__ void cp_async_elem(cplx_t<T>* smem_dst, const cplx_t<T>* gsrc) {
+  if constexpr (sizeof(cplx_t<T>) == 16) {
+    cp_async16(smem_dst, gsrc);
+  } else {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(
+                     static_cast<uint32_t>(__cvta_generic_to_shared(smem_dst))),
+                 "l"(gsrc)
+                 : "memory");
+  }
+}
+
+
+// ---------------------------------------------------------------------------
+// y passes of the y/z kernels with the plane's boundaries folded in (used when
+// both y factors exceed 1).  Rows y of the shared plane sit at offset y * ld,
+// columns c < nz; `rowmask[y]` marks the rows the slab's sphere points touch.
+// ---------------------------------------------------------------------------
+
+// Inverse pass 1 (radix R = L2) over rows sub + j * L1 with the pass-1
+// twiddles; untouched rows are read as zero (they are never zero-filled).
+template <typename T, int R>
+__device__ __forceinline__ void ypass_inv1_R(const int* rowmask, int nz, int L1, int ld, int W, int lim) {
+  cplx_t<T>* sm = smem_c<T>();
+  const int nitems = nz * L1;
+  for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
+    const int sub = it / nz;
+    const int c = it - sub * nz;
+    T re[R], im[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const int y = sub + j * L1;
+      const int off = y * ld + c;
+      if (!QGB_OK_IDX(off, lim, 64)) return;
+      cplx_t<T> v = mk<T>(T(0), T(0));
+      if (rowmask[y]) v = sm[off];
+      re[j] = v.x;
+      im[j] = v.y;
+    }
+    Block<T, R> x;
+    x.load(re, im);
+    x.template run<+1>();
+#pragma unroll
+    for (int j = 1; j < R; ++j) x.template twiddle<+1>(j, sm[W + sub * R + j]);
+    x.store([&](int j, auto value) { sm[(sub + j * L1) * ld + c] = value(); });
+  }
+}
+
+// Inverse pass 2 (radix R = L1) over rows sub * L1 + j, stored straight to the
+// plane in global memory (row stride N2), in the permuted order of the rows.
+template <typename T, int R>
+__device__ __forceinline__ void ypass_inv2_R(cplx_t<T>* __restrict__ out, int N2, int nz, int L2, int ld, int lim) {
+  cplx_t<T>* sm = smem_c<T>();
+  const int nitems = nz * L2;
+  for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
+    const int sub = it / nz;
+    const int c = it - sub * nz;
+    T re[R], im[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const int off = (sub * R + j) * ld + c;
+      if (!QGB_OK_IDX(off, lim, 65)) return;
+      const cplx_t<T> v = sm[off];
+      re[j] = v.x;
+      im[j] = v.y;
+    }
+    Block<T, R> x;
+    x.load(re, im);
+    x.template run<+1>();
+    x.store([&](int j, auto value) { out[static_cast<size_t>(sub * R + j) * N2 + c] = value(); });
+  }
+}
+
+// Forward pass A (radix R = L1) over rows a * L1 + j, read straight from the
+// plane in global memory, times the conjugated pass-A twiddles.
+template <typename T, int R>
+__device__ __forceinline__ void ypass_fwdA_R(const cplx_t<T>* __restrict__ in, int N2, int nz, int L2, int ld, int W,
+                                             int lim) {
+  cplx_t<T>* sm = smem_c<T>();
+  const int nitems = nz * L2;
+  for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
+    const int a = it / nz;
+    const int c = it - a * nz;
+    T re[R], im[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const cplx_t<T> v = in[static_cast<size_t>(a * R + j) * N2 + c];
+      re[j] = v.x;
+      im[j] = v.y;
+    }
+    Block<T, R> x;
+    x.load(re, im);
+    x.template run<-1>();
+#pragma unroll
+    for (int j = 1; j < R; ++j) x.template twiddle<-1>(j, sm[W + a + j * L2]);
+    x.store([&](int j, auto value) {
+      const int off = (a * R + j) * ld + c;
+      if (QGB_OK_IDX(off, lim, 66)) sm[off] = value();
+    });
+  }
+}
+
+// Forward pass B (radix R = L2) over rows sub + j * L1 (natural order out);
+// only the rows the slab's sphere points touch are stored.
+template <typename T, int R>
+__device__ __forceinline__ void ypass_fwdB_R(const int* rowmask, int nz, int L1, int ld, int lim) {
+  cplx_t<T>* sm = smem_c<T>();
+  const int nitems = nz * L1;
+  for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
+    const int sub = it / nz;
+    const int c = it - sub * nz;
+    T re[R], im[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const int off = (sub + j * L1) * ld + c;
+      if (!QGB_OK_IDX(off, lim, 67)) return;
+      const cplx_t<T> v = sm[off];
+      re[j] = v.x;
+      im[j] = v.y;
+    }
+    Block<T, R> x;
+    x.load(re, im);
+    x.template run<-1>();
+    x.store([&](int j, auto value) {
+      if (rowmask[sub + j * L1]) sm[(sub + j * L1) * ld + c] = value();
+    });
+  }
+}
+
+// kind 0: inverse pass 1; 1: inverse pass 2 (to global); 2: forward pass A
+// (from global); 3: forward pass B.  R is the pass's radix.
+template <typename T, int KIND>
+__device__ __forceinline__ void ypass(int R, const int* rowmask, cplx_t<T>* g, int N2, int nz, int L1, int L2,
+                                      int ld, int W, int lim) {
+#define QGB_YP(RR)                                                                  \
+  case RR:                                                                          \
+    if constexpr (KIND == 0) ypass_inv1_R<T, RR>(rowmask, nz, L1, ld, W, lim);      \
+    if constexpr (KIND == 1) ypass_inv2_R<T, RR>(g, N2, nz, L2, ld, lim);           \
+    if constexpr (KIND == 2) ypass_fwdA_R<T, RR>(g, N2, nz, L2, ld, W, lim);        \
+    if constexpr (KIND == 3) ypass_fwdB_R<T, RR>(rowmask, nz, L1, ld, lim);         \
+    break;
+  switch (R) {
+    QGB_YP(2) QGB_YP(3) QGB_YP(4) QGB_YP(5) QGB_YP(6) QGB_YP(7) QGB_YP(8) QGB_YP(9) QGB_YP(10) QGB_YP(12)
+    QGB_YP(14) QGB_YP(15) QGB_YP(16)
+    default: break;
+  }
+#undef QGB_YP
+}
+
+template <typename T>
+__device__ __forceinline__ void body_ifft_yz(const qgb_sphere& s, const LocalParams& lp,
+                                             const cplx_t<T>* __restrict__ C, cplx_t<T>* __restrict__ planes,
+                                             const int slab, const int b, const int k) {
+  using C2 = cplx_t<T>;
+  if (slab >= s.n_slabs[k]) return;
+  const int N1 = s.N[1], N2 = s.N[2], ld = N2 + 1;
+  const int L1y = s.L1[1], L2y = s.L2[1];
+  const bool fold = L1y > 1 && L2y > 1;  // y passes with the plane's boundaries folded in
+  // Shared layout: plane [N1][ld], W_y [N1], W_z [N2], row mask [N1] int.
+  const int lim = N1 * ld, Wy = lim, Wz = Wy + N1;
+  C2* sm = smem_c<T>();
+  int* rowmask = reinterpret_cast<int*>(sm + Wz + N2);
+  const C2* tw = static_cast<const C2*>(s.twiddle);
+  load_twiddles<T>(Wy, tw + s.tw_off[1], N1);
+  load_twiddles<T>(Wz, tw + s.tw_off[2], N2);
+  const C2 zero = mk<T>(T(0), T(0));
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  const int r0 = s.row_start[k * (s.max_slabs + 1) + slab];
+  const int nrows = s.row_start[k * (s.max_slabs + 1) + slab + 1] - r0;
+  const int* rows = s.rows + r0;
+  if (fold) {
+    // Only the touched rows are zero-filled: the first y pass reads the others as zero.
+    for (int y = threadIdx.x; y < N1; y += blockDim.x) rowmask[y] = 0;
+    for (int i = warp; i < nrows; i += nwarps) {
+      const int y = rows[i];
+      if (!QGB_OK_IDX(y, N1, 68)) continue;
+      for (int c = lane; c < N2; c += 32) sm[y * ld + c] = zero;
+    }
+  } else {
+    for (int r = warp; r < N1; r += nwarps)
+      for (int c = lane; c < N2; c += 32) sm[r * ld + c] = zero;
+  }
+  __syncthreads();
+  if (fold) {
+    for (int i = threadIdx.x; i < nrows; i += blockDim.x) {
+      const int y = rows[i];
+      if (QGB_OK_IDX(y, N1, 68)) rowmask[y] = 1;
+    }
+  }
+
+  // Scatter this slab's coefficients (contiguous in the basis) into the plane.
+  const int g0 = s.slab_start[k * (s.max_slabs + 1) + slab];
+  const int g1 = s.slab_start[k * (s.max_slabs + 1) + slab + 1];
+  const C2* Cb = C + (static_cast<size_t>(k) * lp.nb_total + lp.b0 + b) * s.n_tot;
+  const int* yz = s.yz + static_cast<size_t>(k) * s.n_tot;
+  for (int g = g0 + threadIdx.x; g < g1; g += blockDim.x) {
+    if (!QGB_OK_IDX(g, s.n[k], 1)) continue;
+    const int v = yz[g];
+    const int pos = (v >> 16) * ld + (v & 0xFFFF);
+    if (!QGB_OK_IDX(pos, lim, 2) || !QGB_OK_IDX(v & 0xFFFF, N2, 3)) continue;
+    cp_async_elem<T>(sm + pos, Cb + g);
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+
+  // Inverse z-FFT along the rows this slab touches (row stride ld, element
+  // stride 1) and, where the y passes are not folded, the inverse y-FFT along
+  // all N2 columns (column stride 1, element stride ld).
+  if constexpr (sizeof(T) == 8) {  // one copy of the code
+#pragma unroll 1
+    for (int ax = 2; ax >= (fold ? 2 : 1); --ax)
+      fft_axis<T, +1>(0, ax == 2 ? rows : nullptr, ax == 2 ? nrows : N2, ax == 2 ? ld : 1, ax == 2 ? 1 : ld, s.L1[ax],
+                      s.L2[ax], ax == 2 ? Wz : Wy, lim);
+  } else {
+    fft_axis<T, +1>(0, rows, nrows, ld, 1, s.L1[2], s.L2[2], Wz, lim);
+    if (!fold) fft_axis<T, +1>(0, nullptr, N2, 1, ld, L1y, L2y, Wy, lim);
+  }
+  if (!QGB_OK_IDX(plane_index(s, k, b, lp.nb, slab), (long long)s.nk * lp.nb * s.max_slabs, 4)) return;
+  C2* out = planes + plane_index(s, k, b, lp.nb, slab) * (static_cast<size_t>(N1) * N2);
+  if (fold) {
+    // Inverse y-FFT along all N2 columns; its second pass stores the plane.
+    ypass<T, 0>(L2y, rowmask, nullptr, N2, N2, L1y, L2y, ld, Wy, lim);
+    __syncthreads();
+    ypass<T, 1>(L1y, rowmask, out, N2, N2, L1y, L2y, ld, Wy, lim);
+    return;
+  }
+  for (int r = warp; r < N1; r += nwarps)
+    for (int c = lane; c < N2; c += 32) out[r * N2 + c] = sm[r * ld + c];
+}
+
+// The x-pass middle step on one item: inverse L1-point DFT, multiply by V,
+// forward L1-point DFT, forward-pass twiddles; data at sm[p + j*ld], V at
+// Vp[j * vstride] (global or shared), twiddles at sm[Wx + j*L2 + a].
+template <typename T, int R, typename VPtr>
+__device__ __forceinline__ void xmid_item(cplx_t<T>* sm, int p, int ld, VPtr Vp, size_t vstride, int Wx, int L2,
+                                          int a) {
+  using C2 = cplx_t<T>;
+  T re[R], im[R];
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    const C2 v = sm[p + j * ld];
+    re[j] = v.x;
+    im[j] = v.y;
+  }
+  T v[R];
+#pragma unroll
+  for (int j = 0; j < R; ++j) v[j] = Vp[j * vstride];
+  Block<T, R> x;
+  x.load(re, im);
+  x.template run<+1>();
+  x.scale(v);
+  x.template run<-1>();
+  if (L2 > 1) {
+#pragma unroll
+    for (int j = 1; j < R; ++j) x.template twiddle<-1>(j, sm[Wx + j * L2 + a]);
+  }
+  x.store([&](int j, auto value) { sm[p + j * ld] = value(); });
+}
+
+template <typename T, typename VPtr>
+__device__ __forceinline__ void xmid_dispatch(int L1, cplx_t<T>* sm, int p, int ld, VPtr Vp, size_t vstride, int Wx,
+                                              int L2, int a) {
+  switch (L1) {
+    case 1: xmid_item<T, 1>(sm, p, ld, Vp, vstride, Wx, L2, a); break;
+    case 2: xmid_item<T, 2>(sm, p, ld, Vp, vstride, Wx, L2, a); break;
+    case 3: xmid_item<T, 3>(sm, p, ld, Vp, vstride, Wx, L2, a); break;
+    case 4: xmid_item<T, 4>(sm, p, ld, Vp, vstride, Wx, L2, a); break;
+    case 5: xmid_item<T, 5>(sm, p, ld, Vp, vstride, Wx, L2, a); break;
+    case 6: xmid_item<T, 6>(sm, p, ld, Vp, vstride, Wx, L2, a); break;
+    case 7: xmid_item<T, 7>(sm, p, ld, Vp, vstride, Wx, L2, a); break;
+    case 8: xmid_item<T, 8>(sm, p, ld, Vp, vstride, Wx, L2, a); break;
+    case 9: xmid_item<T, 9>(sm, p, ld, Vp, vstride, Wx, L2, a); break;
+    case 10: xmid_item<T, 10>(sm, p, ld, Vp, vstride, Wx, L2, a); break;
+    case 12: xmid_item<T, 12>(sm, p, ld, Vp, vstride, Wx, L2, a); break;
+    case 14: xmid_item<T, 14>(sm, p, ld, Vp, vstride, Wx, L2, a); break;
+    case 15: xmid_item<T, 15>(sm, p, ld, Vp, vstride, Wx, L2, a); break;
+    case 16: xmid_item<T, 16>(sm, p, ld, Vp, vstride, Wx, L2, a); break;
+    default: break;
+  }
+}
+
+// x-pass first inverse pass straight from the slab planes: item (column c,
+// sub) is the L2-point DFT over x = sub + j * L1 (natural order), read from the
+// plane of slab xs[x] (zero where no slab), times the pass-1 twiddles, stored
+// at the same shared rows.  Covers every row, so no zero fill is needed.
+template <typename T, int R>
+__device__ __forceinline__ void xpass_first_R(const cplx_t<T>* __restrict__ base, size_t plane, const int* xs,
+                                              int nz, int L1, int ld, int Wx, int lim) {
+  cplx_t<T>* sm = smem_c<T>();
+  const int nitems = nz * L1;
+  for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
+    const int sub = it / nz;
+    const int c = it - sub * nz;
+    T re[R], im[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const int sl = xs[sub + j * L1];
+      cplx_t<T> v = mk<T>(T(0), T(0));
+      if (sl >= 0) v = base[static_cast<size_t>(sl) * plane + c];
+      re[j] = v.x;
+      im[j] = v.y;
+    }
+    Block<T, R> x;
+    x.load(re, im);
+    x.template run<+1>();
+#pragma unroll
+    for (int j = 1; j < R; ++j) x.template twiddle<+1>(j, sm[Wx + sub * R + j]);
+    x.store([&](int j, auto value) {
+      const int off = (sub + j * L1) * ld + c;
+      if (QGB_OK_IDX(off, lim, 61)) sm[off] = value();
+    });
+  }
+}
+
+// x-pass last forward pass straight to the slab planes: the L2-point DFT over
+// the shared rows sub + j * L1 gives natural x = sub + j * L1; only the rows of
+// a slab (xs[x] >= 0) are stored.
+template <typename T, int R>
+__device__ __forceinline__ void xpass_last_R(cplx_t<T>* __restrict__ base, size_t plane, const int* xs, int nz,
+                                             int L1, int ld, int lim) {
+  cplx_t<T>* sm = smem_c<T>();
+  const int nitems = nz * L1;
+  for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
+    const int sub = it / nz;
+    const int c = it - sub * nz;
+    T re[R], im[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const int off = (sub + j * L1) * ld + c;
+      if (!QGB_OK_IDX(off, lim, 62)) return;
+      const cplx_t<T> v = sm[off];
+      re[j] = v.x;
+      im[j] = v.y;
+    }
+    Block<T, R> x;
+    x.load(re, im);
+    x.template run<-1>();
+    x.store([&](int j, auto value) {
+      const int sl = xs[sub + j * L1];
+      if (sl >= 0) base[static_cast<size_t>(sl) * plane + c] = value();
+    });
+  }
+}
+
+template <typename T, bool FIRST>
+__device__ __forceinline__ void xpass_outer(int R, cplx_t<T>* base, size_t plane, const int* xs, int nz, int L1,
+                                            int ld, int Wx, int lim) {
+#define QGB_XO(RR)                                                   \
+  case RR:                                                           \
+    if constexpr (FIRST)                                             \
+      xpass_first_R<T, RR>(base, plane, xs, nz, L1, ld, Wx, lim);    \
+    else                                                             \
+      xpass_last_R<T, RR>(base, plane, xs, nz, L1, ld, lim);         \
+    break;
+  switch (R) {
+    QGB_XO(2) QGB_XO(3) QGB_XO(4) QGB_XO(5) QGB_XO(6) QGB_XO(7) QGB_XO(8) QGB_XO(9) QGB_XO(10) QGB_XO(12)
+    QGB_XO(14) QGB_XO(15) QGB_XO(16)
+    default: break;
+  }
+#undef QGB_XO
+}
+
+// x-pass of columns [z0, z0 + nz) of y-row r1, with its outer passes on the
+// slab planes: the first inverse pass reads the slab rows from global memory
+// (L2) and the last forward pass stores the slab rows back, so shared memory
+// sees each element in three passes only (no zero fill, staging or write-back).
+// The middle step reads V(r) from global memory (it stays in L2 across the
+// bands).  An axis of a single codelet (L2 = 1) has the middle step alone and
+// is staged.  Shared layout: pencils [N0][nz] complex (threads run along the
+// columns, so rows need no padding), W_x [N0] complex, x -> slab table [N0] int:
+// 75 KB for si64 (96^3) in FP32, so 3 CTAs fit an SM.
+template <typename T>
+__device__ __forceinline__ void body_xpass(const qgb_sphere& s, const LocalParams& lp, cplx_t<T>* __restrict__ planes,
+                                           const int r1, const int b, const int k, const int z0, const int nz) {
+  using C2 = cplx_t<T>;
+  const int N0 = s.N[0], N1 = s.N[1], N2 = s.N[2], ld = nz;
+  const int L1 = s.L1[0], L2 = s.L2[0];
+  const int lim = N0 * ld, Wx = lim;
+  C2* sm = smem_c<T>();
+  int* xs = reinterpret_cast<int*>(sm + Wx + N0);
+  const C2* tw = static_cast<const C2*>(s.twiddle);
+  load_twiddles<T>(Wx, tw + s.tw_off[0], N0);
+  for (int x = threadIdx.x; x < N0; x += blockDim.x) xs[x] = -1;
+  __syncthreads();
+  const int nslabs = s.n_slabs[k];
+  const int* i0 = s.slab_i0 + k * s.max_slabs;
+  for (int sl = threadIdx.x; sl < nslabs; sl += blockDim.x) {
+    const int x = i0[sl];
+    if (QGB_OK_IDX(x, N0, 63)) xs[x] = sl;
+  }
+  __syncthreads();
+  const size_t plane = static_cast<size_t>(N1) * N2;
+  C2* base = planes + plane_index(s, k, b, lp.nb, 0) * plane + static_cast<size_t>(r1) * N2 + z0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  if (L2 > 1) {
+    xpass_outer<T, true>(L2, base, plane, xs, nz, L1, ld, Wx, lim);
+  } else {
+    for (int x = warp; x < N0; x += nwarps) {
+      const int sl = xs[x];
+      for (int c = lane; c < nz; c += 32)
+        sm[x * ld + c] = sl >= 0 ? base[static_cast<size_t>(sl) * plane + c] : mk<T>(T(0), T(0));
+    }
+  }
+  __syncthreads();
+  // V[p0][r1][z0 + c] with p0 = a * L1 + j: j-stride N1 * N2.
+  const T* V = static_cast<const T*>(s.V) + static_cast<size_t>(r1) * N2 + z0;
+  for (int it = threadIdx.x; it < nz * L2; it += blockDim.x) {
+    const int a = it / nz;
+    const int c = it - a * nz;
+    if (!QGB_OK_IDX(c + (a * L1 + L1 - 1) * ld, lim, 7) || !QGB_OK_IDX((L1 - 1) * L2 + a, N0, 9)) continue;
+    xmid_dispatch<T>(L1, sm, c + a * L1 * ld, ld, V + static_cast<size_t>(a) * L1 * N1 * N2 + c,
+                     static_cast<size_t>(N1) * N2, Wx, L2, a);
+  }
+  __syncthreads();
+  if (L2 > 1) {
+    xpass_outer<T, false>(L2, base, plane, xs, nz, L1, ld, Wx, lim);
+  } else {
+    for (int x = warp; x < N0; x += nwarps) {
+      const int sl = xs[x];
+      if (sl >= 0)
+        for (int c = lane; c < nz; c += 32) base[static_cast<size_t>(sl) * plane + c] = sm[x * ld + c];
+    }
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ void body_fft_yz_gather(const qgb_sphere& s, const LocalParams& lp, const cplx_t<T>* C,
+                                                   cplx_t<T>* out, const cplx_t<T>* __restrict__ planes,
+                                                   const int slab, const int b, const int k) {
+  using C2 = cplx_t<T>;
+  const int nslabs = s.n_slabs[k];
+  C2* Ob = out + (static_cast<size_t>(k) * lp.nb_total + lp.b0 + b) * s.n_tot;
+  const bool accumulate = (lp.flags & QGB_ACCUMULATE) != 0;
+  if (slab == 0 && !accumulate) {  // zero the padding entries of this band
+    const int nk_in = s.n[k];
+    for (int g = nk_in + threadIdx.x; g < s.n_tot; g += blockDim.x) Ob[g] = mk<T>(T(0), T(0));
+  }
+  if (slab >= nslabs) return;
+  const int N0 = s.N[0], N1 = s.N[1], N2 = s.N[2], ld = N2 + 1;
+  const int lim = N1 * ld, Wy = lim, Wz = Wy + N1;
+  C2* sm = smem_c<T>();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  if (!QGB_OK_IDX(plane_index(s, k, b, lp.nb, slab), (long long)s.nk * lp.nb * s.max_slabs, 4)) return;
+  const C2* in = planes + plane_index(s, k, b, lp.nb, slab) * (static_cast<size_t>(N1) * N2);
+  const int L1y = s.L1[1], L2y = s.L2[1];
+  const int r0 = s.row_start[k * (s.max_slabs + 1) + slab];
+  const int nrows = s.row_start[k * (s.max_slabs + 1) + slab + 1] - r0;
+  const C2* tw = static_cast<const C2*>(s.twiddle);
+  const bool fold = L1y > 1 && L2y > 1;
+  if (fold) {
+    // The first forward y pass reads the plane from global memory; the second
+    // stores only the rows the z-FFT and the gather use.
+    int* rowmask = reinterpret_cast<int*>(sm + Wz + N2);
+    for (int y = threadIdx.x; y < N1; y += blockDim.x) rowmask[y] = 0;
+    load_twiddles<T>(Wy, tw + s.tw_off[1], N1);
+    load_twiddles<T>(Wz, tw + s.tw_off[2], N2);
+    __syncthreads();
+    for (int i = threadIdx.x; i < nrows; i += blockDim.x) {
+      const int y = s.rows[r0 + i];
+      if (QGB_OK_IDX(y, N1, 68)) rowmask[y] = 1;
+    }
+    ypass<T, 2>(L1y, rowmask, const_cast<C2*>(in), N2, N2, L1y, L2y, ld, Wy, lim);
+    __syncthreads();
+    ypass<T, 3>(L2y, rowmask, nullptr, N2, N2, L1y, L2y, ld, Wy, lim);
+    __syncthreads();
+  } else {
+    // Stage the plane asynchronously (padded rows are 8-byte aligned only, so one
+    // element per copy), then the twiddles while the copies are in flight.
+    for (int r = warp; r < N1; r += nwarps)
+      for (int c = lane; c < N2; c += 32) cp_async_elem<T>(sm + r * ld + c, in + r * N2 + c);
+    cp_async_commit();
+    load_twiddles<T>(Wy, tw + s.tw_off[1], N1);
+    load_twiddles<T>(Wz, tw + s.tw_off[2], N2);
+    cp_async_wait<0>();
+    __syncthreads();
+  }
+  // Forward y-FFT along all columns (unless folded above), then the forward
+  // z-FFT along the touched rows.
+  if constexpr (sizeof(T) == 8) {
+#pragma unroll 1
+    for (int ax = fold ? 2 : 1; ax <= 2; ++ax)
+      fft_axis<T, -1>(0, ax == 2 ? s.rows + r0 : nullptr, ax == 2 ? nrows : N2, ax == 2 ? ld : 1, ax == 2 ? 1 : ld,
+                      s.L1[ax], s.L2[ax], ax == 2 ? Wz : Wy, lim);
+  } else {
+    if (!fold) fft_axis<T, -1>(0, nullptr, N2, 1, ld, L1y, L2y, Wy, lim);
+    fft_axis<T, -1>(0, s.rows + r0, nrows, ld, 1, s.L1[2], s.L2[2], Wz, lim);
+  }
+
+  const int g0 = s.slab_start[k * (s.max_slabs + 1) + slab];
+  const int g1 = s.slab_start[k * (s.max_slabs + 1) + slab + 1];
+  const C2* Cb = C + (static_cast<size_t>(k) * lp.nb_total + lp.b0 + b) * s.n_tot;
+  const int* yz = s.yz + static_cast<size_t>(k) * s.n_tot;
+  const T invN = T(1) / (T(N0) * T(N1) * T(N2));
+  const bool add_ke = (lp.flags & QGB_ADD_KE) != 0;
+  const T* ke = static_cast<const T*>(s.ke) + static_cast<size_t>(k) * s.n_tot;
+  for (int g = g0 + threadIdx.x; g < g1; g += blockDim.x) {
+    if (!QGB_OK_IDX(g, s.n[k], 1)) continue;
+    const int v = yz[g];
+    const int pos = (v >> 16) * ld + (v & 0xFFFF);
+    if (!QGB_OK_IDX(pos, lim, 2)) continue;
+    const C2 f = sm[pos];
+    T xr = f.x * invN, xi = f.y * invN;
+    if (add_ke) {
+      const C2 c = Cb[g];
+      const T e = ke[g];
+      xr = e * c.x + xr;
+      xi = e * c.y + xi;
+    }
+    if (accumulate) {
+      const C2 o = Ob[g];
+      xr += o.x;
+      xi += o.y;
+    }
+    Ob[g] = mk<T>(xr, xi);
+  }
+}
+
+
+// ---------------------------------------------------------------------------
+// Kernels: one sphere (grid = work units of that sphere) ...
+// ---------------------------------------------------------------------------
+
+// FP32: 80 registers, three CTAs of 256 threads an SM; FP64 (block fixed point,
+// 128 registers): up to 512 threads an SM, see pick_threads.
+template <typename T> constexpr int kMaxThreadsYZ = sizeof(T) == 4 ? 256 : 512;
+template <typename T> constexpr int kCtasX = sizeof(T) == 4 ? 3 : 2;
+
+template <typename T>
+__global__ void __launch_bounds__(kMaxThreadsYZ<T>, sizeof(T) == 4 ? 3 : 1) k_ifft_yz(const qgb_sphere s, LocalParams lp,
+                                                              const cplx_t<T>* __restrict__ C,
+                                                              cplx_t<T>* __restrict__ planes) {
+  body_ifft_yz<T>(s, lp, C, planes, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+// The columns of a y-row in `zs` parts of `nzp`.
+template <typename T>
+__global__ void __launch_bounds__(kThreads, kCtasX<T>) k_xpass(const qgb_sphere s, LocalParams lp,
+                                                            cplx_t<T>* __restrict__ planes, int zs, int nzp) {
+  const int r1 = blockIdx.x / zs, z0 = (blockIdx.x - r1 * zs) * nzp;
+  const int nz = min(nzp, s.N[2] - z0);
+  if (nz > 0) body_xpass<T>(s, lp, planes, r1, blockIdx.y, blockIdx.z, z0, nz);
+}
+
+// C and out may alias (in-place apply): no __restrict__ on them.
+template <typename T>
+__global__ void __launch_bounds__(kMaxThreadsYZ<T>, sizeof(T) == 4 ? 3 : 1) k_fft_yz_gather(const qgb_sphere s, LocalParams lp,
+                                                                    const cplx_t<T>* C, cplx_t<T>* out,
+                                                                    const cplx_t<T>* __restrict__ planes) {
+  body_fft_yz_gather<T>(s, lp, C, out, planes, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+
+// ---------------------------------------------------------------------------
+// Launches of one precision (instantiated in local_f32.cu and local_f64.cu)
+// ---------------------------------------------------------------------------
+
+inline size_t yz_smem_bytes(const qgb_sphere& s, size_t e) {
+  return (static_cast<size_t>(s.N[1]) * (s.N[2] + 1) + s.N[1] + s.N[2]) * e + s.N[1] * sizeof(int);
+}
+inline size_t x_smem_bytes(const qgb_sphere& s, int nz, size_t e) {
+  return (static_cast<size_t>(s.N[0]) * nz + s.N[0]) * e + s.N[0] * sizeof(int);
+}
+
+constexpr size_t kSmemPerSm = 227 * 1024;
+
+// CTA size of the FP64 kernels, whose passes have a few items per thread.  The
+// cost of a CTA size is the thread-rounds of the two heavy passes (a and b
+// items), more if the SM's CTAs (128 registers a thread, `smem` bytes each) have
+// fewer than 512 threads to hide the latencies of the integer pipes.
+inline double threads_cost(int t, int a, int b, size_t smem) {
+  const int ctas = std::max(1, static_cast<int>(std::min<size_t>(512 / t, (kSmemPerSm + 1024) / (smem + 1024))));
+  const int rounds = (a + t - 1) / t + (b + t - 1) / t;
+  return static_cast<double>(rounds) * t * std::pow(512.0 / (ctas * t), 0.7);
+}
+inline int pick_threads(int a, int b, size_t smem, int max_threads, double* cost = nullptr) {
+  int best = 128;
+  double best_cost = 1e30;
+  for (int t = 96; t <= max_threads; t += 32) {
+    const double c = threads_cost(t, a, b, smem);
+    if (c < best_cost * 0.999) {
+      best_cost = c;
+      best = t;
+    }
+  }
+  if (cost) *cost = best_cost;
+  return best;
+}
+
+template <typename T> int threads_yz(const qgb_sphere& s) {
+  if (sizeof(T) == 4) return kThreads;
+  return pick_threads(s.N[2] * s.L1[1], s.N[2] * s.L2[1], yz_smem_bytes(s, 16), kMaxThreadsYZ<T>);
+}
+
+// The x-pass takes a y-row's columns in `zs` parts: FP32 whole rows while two
+// CTAs fit an SM, FP64 the split and CTA size that cost the least per column
+// (for si64 three parts of 32 columns, four CTAs of 128 threads an SM).
+template <typename T> void x_split(const qgb_sphere& s, int* zs, int* threads) {
+  const int N2 = s.N[2];
+  *zs = 1;
+  *threads = kThreads;
+  if (sizeof(T) == 4) {
+    while (*zs < N2 && x_smem_bytes(s, (N2 + *zs - 1) / *zs, 8) > kSmemPerSm / 2 - 1024) ++*zs;
+    return;
+  }
+  double best = 1e30;
+  for (int z = 1; z <= 8; ++z) {
+    const int nz = (N2 + z - 1) / z;
+    const size_t smem = x_smem_bytes(s, nz, 16);
+    if ((nz < 16 && z > 1) || smem > kSmemPerSm) continue;
+    double c;
+    const int t = pick_threads(nz * s.L1[0], nz * s.L2[0], smem, kThreads, &c);
+    c *= z;                           // parts per row
+    c += 0.5 * z * s.N[0];            // tables of each CTA
+    if (c < best) {
+      best = c;
+      *zs = z;
+      *threads = t;
+    }
+  }
+}
+
+template <typename T>
+int launch_ifft_yz(const qgb_sphere& s, const LocalParams& lp, const void* C, void* planes, cudaStream_t st) {
+  const size_t smem = yz_smem_bytes(s, sizeof(cplx_t<T>));
+  if (int rc = raise_smem_limit(k_ifft_yz<T>, smem)) return rc;
+  k_ifft_yz<T><<<dim3(s.max_slabs, lp.nb, s.nk), threads_yz<T>(s), smem, st>>>(
+      s, lp, static_cast<const cplx_t<T>*>(C), static_cast<cplx_t<T>*>(planes));
+  QGB_LAUNCH_CHECK("k_ifft_yz");
+  return QGB_OK;
+}
+
+template <typename T>
+int launch_chunk(const qgb_sphere& s, const LocalParams& lp, const void* C, void* out, void* planes, cudaStream_t st,
+                 cudaEvent_t gather_after) {
+  using C2 = cplx_t<T>;
+  int rc;
+  if ((rc = launch_ifft_yz<T>(s, lp, C, planes, st))) return rc;
+  int zs, tx;
+  x_split<T>(s, &zs, &tx);
+  const int nzp = (s.N[2] + zs - 1) / zs;
+  const size_t smx = x_smem_bytes(s, nzp, sizeof(C2));
+  if ((rc = raise_smem_limit(k_xpass<T>, smx))) return rc;
+  k_xpass<T><<<dim3(s.N[1] * zs, lp.nb, s.nk), tx, smx, st>>>(s, lp, static_cast<C2*>(planes), zs, nzp);
+  QGB_LAUNCH_CHECK("k_xpass");
+  if (gather_after) QGB_CUDA_CHECK(cudaStreamWaitEvent(st, gather_after, 0));
+  const size_t smem = yz_smem_bytes(s, sizeof(C2));
+  if ((rc = raise_smem_limit(k_fft_yz_gather<T>, smem))) return rc;
+  k_fft_yz_gather<T><<<dim3(s.max_slabs, lp.nb, s.nk), threads_yz<T>(s), smem, st>>>(
+      s, lp, static_cast<const C2*>(C), static_cast<C2*>(out), static_cast<const C2*>(planes));
+  QGB_LAUNCH_CHECK("k_fft_yz_gather");
+  return QGB_OK;
+}
+
+#ifdef QGB_DEBUG_CHECKS
+// Debug builds: add this translation unit's first recorded range violation
+// (site, index, limit, packed block index; site 0 = none) to out4 if that is
+// still empty, and clear it.
+static int unit_violation(unsigned long long* out4) {
+  unsigned long long v[4];
+  QGB_CUDA_CHECK(cudaMemcpyFromSymbol(v, g_qgb_violation, sizeof(v)));
+  const unsigned long long zero[4] = {0, 0, 0, 0};
+  QGB_CUDA_CHECK(cudaMemcpyToSymbol(g_qgb_violation, zero, sizeof(zero)));
+  if (out4[0] == 0)
+    for (int i = 0; i < 4; ++i) out4[i] = v[i];
+  return QGB_OK;
+}
+#endif
+
+}  // namespace qgb
