@@ -29,6 +29,15 @@ namespace qgb {
 
 extern __shared__ __align__(16) unsigned char qgb_smem[];
 
+// n / d by a multiplication, for n d < 2^32 and d >= 2 (a pass's items over its
+// columns; the compiler's own division by a run-time d is some 20 instructions
+// per item).
+struct FastDiv {
+  unsigned d, m;
+  __device__ __forceinline__ explicit FastDiv(int divisor) : d(divisor), m(divisor > 1 ? 0xFFFFFFFFu / divisor + 1 : 0) {}
+  __device__ __forceinline__ int quot(int n) const { return d > 1 ? static_cast<int>(__umulhi(n, m)) : n; }
+};
+
 template <typename T> __device__ __forceinline__ cplx_t<T>* smem_c() {
   return reinterpret_cast<cplx_t<T>*>(qgb_smem);
 }
@@ -76,8 +85,9 @@ struct Pass {
 template <typename T, int S, int R>
 __device__ __forceinline__ void run_pass_R(const Pass ps) {
   const int nitems = ps.nbatch * ps.nsub;
+  const FastDiv div(ps.nbatch);
   for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
-    const int sub = it / ps.nbatch;
+    const int sub = div.quot(it);
     const int b = it - sub * ps.nbatch;
     const int boff = (ps.bmap != nullptr ? __ldg(ps.bmap + b) : b) * ps.bstride;
     codelet_inplace<T, S, R>(ps.base + boff + sub * ps.sstride, ps.estride,

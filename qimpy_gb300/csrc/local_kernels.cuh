@@ -68,8 +68,9 @@ template <typename T, int R>
 __device__ __forceinline__ void ypass_inv1_R(const int* rowmask, int nz, int L1, int ld, int W, int lim) {
   cplx_t<T>* sm = smem_c<T>();
   const int nitems = nz * L1;
+  const FastDiv div(nz);
   for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
-    const int sub = it / nz;
+    const int sub = div.quot(it);
     const int c = it - sub * nz;
     T re[R], im[R];
 #pragma unroll
@@ -97,8 +98,9 @@ template <typename T, int R>
 __device__ __forceinline__ void ypass_inv2_R(cplx_t<T>* __restrict__ out, int N2, int nz, int L2, int ld, int lim) {
   cplx_t<T>* sm = smem_c<T>();
   const int nitems = nz * L2;
+  const FastDiv div(nz);
   for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
-    const int sub = it / nz;
+    const int sub = div.quot(it);
     const int c = it - sub * nz;
     T re[R], im[R];
 #pragma unroll
@@ -112,7 +114,7 @@ __device__ __forceinline__ void ypass_inv2_R(cplx_t<T>* __restrict__ out, int N2
     Block<T, R> x;
     x.load(re, im);
     x.template run<+1>();
-    x.store([&](int j, auto value) { out[static_cast<size_t>(sub * R + j) * N2 + c] = value(); });
+    x.store([&](int j, auto value) { out[static_cast<unsigned>((sub * R + j) * N2 + c)] = value(); });
   }
 }
 
@@ -123,13 +125,14 @@ __device__ __forceinline__ void ypass_fwdA_R(const cplx_t<T>* __restrict__ in, i
                                              int lim) {
   cplx_t<T>* sm = smem_c<T>();
   const int nitems = nz * L2;
+  const FastDiv div(nz);
   for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
-    const int a = it / nz;
+    const int a = div.quot(it);
     const int c = it - a * nz;
     T re[R], im[R];
 #pragma unroll
     for (int j = 0; j < R; ++j) {
-      const cplx_t<T> v = in[static_cast<size_t>(a * R + j) * N2 + c];
+      const cplx_t<T> v = in[static_cast<unsigned>((a * R + j) * N2 + c)];
       re[j] = v.x;
       im[j] = v.y;
     }
@@ -151,8 +154,9 @@ template <typename T, int R>
 __device__ __forceinline__ void ypass_fwdB_R(const int* rowmask, int nz, int L1, int ld, int lim) {
   cplx_t<T>* sm = smem_c<T>();
   const int nitems = nz * L1;
+  const FastDiv div(nz);
   for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
-    const int sub = it / nz;
+    const int sub = div.quot(it);
     const int c = it - sub * nz;
     T re[R], im[R];
 #pragma unroll
@@ -278,7 +282,7 @@ __device__ __forceinline__ void body_ifft_yz(const qgb_sphere& s, const LocalPar
 // forward L1-point DFT, forward-pass twiddles; data at sm[p + j*ld], V at
 // Vp[j * vstride] (global or shared), twiddles at sm[Wx + j*L2 + a].
 template <typename T, int R, typename VPtr>
-__device__ __forceinline__ void xmid_item(cplx_t<T>* sm, int p, int ld, VPtr Vp, size_t vstride, int Wx, int L2,
+__device__ __forceinline__ void xmid_item(cplx_t<T>* sm, int p, int ld, VPtr Vp, unsigned vstride, int Wx, int L2,
                                           int a) {
   using C2 = cplx_t<T>;
   T re[R], im[R];
@@ -304,7 +308,7 @@ __device__ __forceinline__ void xmid_item(cplx_t<T>* sm, int p, int ld, VPtr Vp,
 }
 
 template <typename T, typename VPtr>
-__device__ __forceinline__ void xmid_dispatch(int L1, cplx_t<T>* sm, int p, int ld, VPtr Vp, size_t vstride, int Wx,
+__device__ __forceinline__ void xmid_dispatch(int L1, cplx_t<T>* sm, int p, int ld, VPtr Vp, unsigned vstride, int Wx,
                                               int L2, int a) {
   switch (L1) {
     case 1: xmid_item<T, 1>(sm, p, ld, Vp, vstride, Wx, L2, a); break;
@@ -327,22 +331,23 @@ __device__ __forceinline__ void xmid_dispatch(int L1, cplx_t<T>* sm, int p, int 
 
 // x-pass first inverse pass straight from the slab planes: item (column c,
 // sub) is the L2-point DFT over x = sub + j * L1 (natural order), read from the
-// plane of slab xs[x] (zero where no slab), times the pass-1 twiddles, stored
+// planes at offset xs[x] (zero where no slab), times the pass-1 twiddles, stored
 // at the same shared rows.  Covers every row, so no zero fill is needed.
 template <typename T, int R>
-__device__ __forceinline__ void xpass_first_R(const cplx_t<T>* __restrict__ base, size_t plane, const int* xs,
+__device__ __forceinline__ void xpass_first_R(const cplx_t<T>* __restrict__ base, const int* xs,
                                               int nz, int L1, int ld, int Wx, int lim) {
   cplx_t<T>* sm = smem_c<T>();
   const int nitems = nz * L1;
+  const FastDiv div(nz);
   for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
-    const int sub = it / nz;
+    const int sub = div.quot(it);
     const int c = it - sub * nz;
     T re[R], im[R];
 #pragma unroll
     for (int j = 0; j < R; ++j) {
-      const int sl = xs[sub + j * L1];
+      const int o = xs[sub + j * L1];
       cplx_t<T> v = mk<T>(T(0), T(0));
-      if (sl >= 0) v = base[static_cast<size_t>(sl) * plane + c];
+      if (o >= 0) v = base[static_cast<unsigned>(o + c)];
       re[j] = v.x;
       im[j] = v.y;
     }
@@ -362,12 +367,13 @@ __device__ __forceinline__ void xpass_first_R(const cplx_t<T>* __restrict__ base
 // the shared rows sub + j * L1 gives natural x = sub + j * L1; only the rows of
 // a slab (xs[x] >= 0) are stored.
 template <typename T, int R>
-__device__ __forceinline__ void xpass_last_R(cplx_t<T>* __restrict__ base, size_t plane, const int* xs, int nz,
+__device__ __forceinline__ void xpass_last_R(cplx_t<T>* __restrict__ base, const int* xs, int nz,
                                              int L1, int ld, int lim) {
   cplx_t<T>* sm = smem_c<T>();
   const int nitems = nz * L1;
+  const FastDiv div(nz);
   for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
-    const int sub = it / nz;
+    const int sub = div.quot(it);
     const int c = it - sub * nz;
     T re[R], im[R];
 #pragma unroll
@@ -382,21 +388,21 @@ __device__ __forceinline__ void xpass_last_R(cplx_t<T>* __restrict__ base, size_
     x.load(re, im);
     x.template run<-1>();
     x.store([&](int j, auto value) {
-      const int sl = xs[sub + j * L1];
-      if (sl >= 0) base[static_cast<size_t>(sl) * plane + c] = value();
+      const int o = xs[sub + j * L1];
+      if (o >= 0) base[static_cast<unsigned>(o + c)] = value();
     });
   }
 }
 
 template <typename T, bool FIRST>
-__device__ __forceinline__ void xpass_outer(int R, cplx_t<T>* base, size_t plane, const int* xs, int nz, int L1,
+__device__ __forceinline__ void xpass_outer(int R, cplx_t<T>* base, const int* xs, int nz, int L1,
                                             int ld, int Wx, int lim) {
 #define QGB_XO(RR)                                                   \
   case RR:                                                           \
     if constexpr (FIRST)                                             \
-      xpass_first_R<T, RR>(base, plane, xs, nz, L1, ld, Wx, lim);    \
+      xpass_first_R<T, RR>(base, xs, nz, L1, ld, Wx, lim);    \
     else                                                             \
-      xpass_last_R<T, RR>(base, plane, xs, nz, L1, ld, lim);         \
+      xpass_last_R<T, RR>(base, xs, nz, L1, ld, lim);         \
     break;
   switch (R) {
     QGB_XO(2) QGB_XO(3) QGB_XO(4) QGB_XO(5) QGB_XO(6) QGB_XO(7) QGB_XO(8) QGB_XO(9) QGB_XO(10) QGB_XO(12)
@@ -406,8 +412,8 @@ __device__ __forceinline__ void xpass_outer(int R, cplx_t<T>* base, size_t plane
 #undef QGB_XO
 }
 
-// x-pass of columns [z0, z0 + nz) of y-row r1, with its outer passes on the
-// slab planes: the first inverse pass reads the slab rows from global memory
+// x-pass of the columns [c0, c0 + nz) of the N1 N2 (y, z) positions of a plane,
+// with its outer passes on the slab planes: the first inverse pass reads the slab rows from global memory
 // (L2) and the last forward pass stores the slab rows back, so shared memory
 // sees each element in three passes only (no zero fill, staging or write-back).
 // The middle step reads V(r) from global memory (it stays in L2 across the
@@ -417,7 +423,7 @@ __device__ __forceinline__ void xpass_outer(int R, cplx_t<T>* base, size_t plane
 // 75 KB for si64 (96^3) in FP32, so 3 CTAs fit an SM.
 template <typename T>
 __device__ __forceinline__ void body_xpass(const qgb_sphere& s, const LocalParams& lp, cplx_t<T>* __restrict__ planes,
-                                           const int r1, const int b, const int k, const int z0, const int nz) {
+                                           const int b, const int k, const int c0, const int nz) {
   using C2 = cplx_t<T>;
   const int N0 = s.N[0], N1 = s.N[1], N2 = s.N[2], ld = nz;
   const int L1 = s.L1[0], L2 = s.L2[0];
@@ -432,39 +438,39 @@ __device__ __forceinline__ void body_xpass(const qgb_sphere& s, const LocalParam
   const int* i0 = s.slab_i0 + k * s.max_slabs;
   for (int sl = threadIdx.x; sl < nslabs; sl += blockDim.x) {
     const int x = i0[sl];
-    if (QGB_OK_IDX(x, N0, 63)) xs[x] = sl;
+    if (QGB_OK_IDX(x, N0, 63)) xs[x] = sl * N1 * N2;
   }
   __syncthreads();
   const size_t plane = static_cast<size_t>(N1) * N2;
-  C2* base = planes + plane_index(s, k, b, lp.nb, 0) * plane + static_cast<size_t>(r1) * N2 + z0;
+  C2* base = planes + plane_index(s, k, b, lp.nb, 0) * plane + c0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   if (L2 > 1) {
-    xpass_outer<T, true>(L2, base, plane, xs, nz, L1, ld, Wx, lim);
+    xpass_outer<T, true>(L2, base, xs, nz, L1, ld, Wx, lim);
   } else {
     for (int x = warp; x < N0; x += nwarps) {
-      const int sl = xs[x];
-      for (int c = lane; c < nz; c += 32)
-        sm[x * ld + c] = sl >= 0 ? base[static_cast<size_t>(sl) * plane + c] : mk<T>(T(0), T(0));
+      const int o = xs[x];
+      for (int c = lane; c < nz; c += 32) sm[x * ld + c] = o >= 0 ? base[o + c] : mk<T>(T(0), T(0));
     }
   }
   __syncthreads();
-  // V[p0][r1][z0 + c] with p0 = a * L1 + j: j-stride N1 * N2.
-  const T* V = static_cast<const T*>(s.V) + static_cast<size_t>(r1) * N2 + z0;
+  // V[p0][c0 + c] with p0 = a * L1 + j: j-stride N1 * N2.
+  const T* V = static_cast<const T*>(s.V) + c0;
+  const FastDiv div(nz);
   for (int it = threadIdx.x; it < nz * L2; it += blockDim.x) {
-    const int a = it / nz;
+    const int a = div.quot(it);
     const int c = it - a * nz;
     if (!QGB_OK_IDX(c + (a * L1 + L1 - 1) * ld, lim, 7) || !QGB_OK_IDX((L1 - 1) * L2 + a, N0, 9)) continue;
-    xmid_dispatch<T>(L1, sm, c + a * L1 * ld, ld, V + static_cast<size_t>(a) * L1 * N1 * N2 + c,
-                     static_cast<size_t>(N1) * N2, Wx, L2, a);
+    xmid_dispatch<T>(L1, sm, c + a * L1 * ld, ld, V + static_cast<unsigned>(a * L1 * N1 * N2 + c),
+                     N1 * N2, Wx, L2, a);
   }
   __syncthreads();
   if (L2 > 1) {
-    xpass_outer<T, false>(L2, base, plane, xs, nz, L1, ld, Wx, lim);
+    xpass_outer<T, false>(L2, base, xs, nz, L1, ld, Wx, lim);
   } else {
     for (int x = warp; x < N0; x += nwarps) {
-      const int sl = xs[x];
-      if (sl >= 0)
-        for (int c = lane; c < nz; c += 32) base[static_cast<size_t>(sl) * plane + c] = sm[x * ld + c];
+      const int o = xs[x];
+      if (o >= 0)
+        for (int c = lane; c < nz; c += 32) base[o + c] = sm[x * ld + c];
     }
   }
 }
@@ -566,30 +572,29 @@ __device__ __forceinline__ void body_fft_yz_gather(const qgb_sphere& s, const Lo
 // Kernels: one sphere (grid = work units of that sphere) ...
 // ---------------------------------------------------------------------------
 
-// FP32: 80 registers, three CTAs of 256 threads an SM; FP64 (block fixed point,
-// 128 registers): up to 512 threads an SM, see pick_threads.
-template <typename T> constexpr int kMaxThreadsYZ = sizeof(T) == 4 ? 256 : 512;
+// FP32 takes 80 registers (768 threads an SM), FP64 (block fixed point) 128 (512
+// threads); the CTA sizes follow the grid, see launch_cost.
+template <typename T> constexpr int kMaxThreadsYZ = sizeof(T) == 4 ? 384 : 512;
 template <typename T> constexpr int kCtasX = sizeof(T) == 4 ? 3 : 2;
 
 template <typename T>
-__global__ void __launch_bounds__(kMaxThreadsYZ<T>, sizeof(T) == 4 ? 3 : 1) k_ifft_yz(const qgb_sphere s, LocalParams lp,
+__global__ void __launch_bounds__(kMaxThreadsYZ<T>, sizeof(T) == 4 ? 2 : 1) k_ifft_yz(const qgb_sphere s, LocalParams lp,
                                                               const cplx_t<T>* __restrict__ C,
                                                               cplx_t<T>* __restrict__ planes) {
   body_ifft_yz<T>(s, lp, C, planes, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
-// The columns of a y-row in `zs` parts of `nzp`.
+// A tile of `nc` columns per CTA.
 template <typename T>
 __global__ void __launch_bounds__(kThreads, kCtasX<T>) k_xpass(const qgb_sphere s, LocalParams lp,
-                                                            cplx_t<T>* __restrict__ planes, int zs, int nzp) {
-  const int r1 = blockIdx.x / zs, z0 = (blockIdx.x - r1 * zs) * nzp;
-  const int nz = min(nzp, s.N[2] - z0);
-  if (nz > 0) body_xpass<T>(s, lp, planes, r1, blockIdx.y, blockIdx.z, z0, nz);
+                                                            cplx_t<T>* __restrict__ planes, int nc) {
+  const int c0 = blockIdx.x * nc;
+  body_xpass<T>(s, lp, planes, blockIdx.y, blockIdx.z, c0, min(nc, s.N[1] * s.N[2] - c0));
 }
 
 // C and out may alias (in-place apply): no __restrict__ on them.
 template <typename T>
-__global__ void __launch_bounds__(kMaxThreadsYZ<T>, sizeof(T) == 4 ? 3 : 1) k_fft_yz_gather(const qgb_sphere s, LocalParams lp,
+__global__ void __launch_bounds__(kMaxThreadsYZ<T>, sizeof(T) == 4 ? 2 : 1) k_fft_yz_gather(const qgb_sphere s, LocalParams lp,
                                                                     const cplx_t<T>* C, cplx_t<T>* out,
                                                                     const cplx_t<T>* __restrict__ planes) {
   body_fft_yz_gather<T>(s, lp, C, out, planes, blockIdx.x, blockIdx.y, blockIdx.z);
@@ -608,58 +613,67 @@ inline size_t x_smem_bytes(const qgb_sphere& s, int nz, size_t e) {
 
 constexpr size_t kSmemPerSm = 227 * 1024;
 
-// CTA size of the FP64 kernels, whose passes have a few items per thread.  The
-// cost of a CTA size is the thread-rounds of the two heavy passes (a and b
-// items), more if the SM's CTAs (128 registers a thread, `smem` bytes each) have
-// fewer than 512 threads to hide the latencies of the integer pipes.
-inline double threads_cost(int t, int a, int b, size_t smem) {
-  const int ctas = std::max(1, static_cast<int>(std::min<size_t>(512 / t, (kSmemPerSm + 1024) / (smem + 1024))));
-  const int rounds = (a + t - 1) / t + (b + t - 1) / t;
-  return static_cast<double>(rounds) * t * std::pow(512.0 / (ctas * t), 0.7);
+// Relative cost of a launch: `ctas_total` CTAs of t threads and `smem` bytes,
+// each doing `work` thread-rounds (a round counts its codelet's elements).  An
+// SM holds 768 threads of 80 registers in FP32, 512 of 128 in FP64; wide CTAs
+// wait longer at their barriers; a launch of few CTAs takes whole waves.
+template <typename T> double launch_cost(double ctas_total, int t, size_t smem, double work) {
+  const int resident = sizeof(T) == 4 ? 768 : 512;
+  const int ctas = std::max(1, static_cast<int>(std::min<size_t>(resident / t, (kSmemPerSm + 1024) / (smem + 1024))));
+  double waves = std::max(1.0, ctas_total / (152.0 * ctas));
+  if (waves < 8.0) waves = std::ceil(waves);
+  const double on_sm = std::min<double>(ctas, std::ceil(ctas_total / 152.0)) * t;
+  return waves * work * (1.0 + 0.0006 * t) * std::max(0.5, std::sqrt(on_sm / resident));
 }
-inline int pick_threads(int a, int b, size_t smem, int max_threads, double* cost = nullptr) {
-  int best = 128;
-  double best_cost = 1e30;
-  for (int t = 96; t <= max_threads; t += 32) {
-    const double c = threads_cost(t, a, b, smem);
-    if (c < best_cost * 0.999) {
-      best_cost = c;
-      best = t;
+
+// CTA size of the y/z kernels: the one whose passes (y: N2 L1 items of radix L2
+// and N2 L2 of L1; z: the touched rows, on average 0.8 of the most) fill their
+// rounds.  Measured against 256 threads (FP32; 36^3 in FP64 against 224), us: 36^3,
+// 144 bands, 43 -> 28 (FP64 144 -> 110); 72^3, 800 bands, inverse 513 -> 450.
+template <typename T> int threads_yz(const qgb_sphere& s, int nb) {
+  const size_t smem = yz_smem_bytes(s, sizeof(cplx_t<T>));
+  const int zrows = std::max(1, s.max_rows * 4 / 5);
+  double best = 1e30;
+  int threads = 128;
+  for (int t = 96; t <= kMaxThreadsYZ<T>; t += 32) {
+    auto rounds = [t](int items) { return (items + t - 1) / t; };
+    const double work = rounds(s.N[2] * s.L1[1]) * s.L2[1] + rounds(s.N[2] * s.L2[1]) * s.L1[1] +
+                        rounds(zrows * s.L1[2]) * s.L2[2] + rounds(zrows * s.L2[2]) * s.L1[2] + 8.0;
+    const double cost = launch_cost<T>(static_cast<double>(s.max_slabs) * nb * s.nk, t, smem, work);
+    if (cost < best * 0.999) {
+      best = cost;
+      threads = t;
     }
   }
-  if (cost) *cost = best_cost;
-  return best;
+  return threads;
 }
 
-template <typename T> int threads_yz(const qgb_sphere& s) {
-  if (sizeof(T) == 4) return kThreads;
-  return pick_threads(s.N[2] * s.L1[1], s.N[2] * s.L2[1], yz_smem_bytes(s, 16), kMaxThreadsYZ<T>);
-}
-
-// The x-pass takes a y-row's columns in `zs` parts: FP32 whole rows while two
-// CTAs fit an SM, FP64 the split and CTA size that cost the least per column
-// (for si64 three parts of 32 columns, four CTAs of 128 threads an SM).
-template <typename T> void x_split(const qgb_sphere& s, int* zs, int* threads) {
-  const int N2 = s.N[2];
-  *zs = 1;
-  *threads = kThreads;
-  if (sizeof(T) == 4) {
-    while (*zs < N2 && x_smem_bytes(s, (N2 + *zs - 1) / *zs, 8) > kSmemPerSm / 2 - 1024) ++*zs;
-    return;
-  }
+// Tile of columns and CTA size of the x-pass.  A plane's N1 N2 columns are one
+// contiguous range, so a tile need not be a y-row: it is the one for which the
+// passes fill their rounds of the CTA's threads (nc L1 items of radix L2 twice,
+// nc L2 items of radix L1 in both directions), by launch_cost; a CTA's tables
+// and barriers count 8 and its share of them.  Tiles below 32 columns (256 B of
+// a row) load worse.
+// Measured against whole y-rows (us, FP32): si64 (96^3, 160 bands; a row of 96 in
+// 5 + 3 rounds of 256 threads, a tile of 32 in 3 + 2 full ones of 128) 436 ->
+// 416; 36^3, 144 bands (216 items a row) 38 -> 25; 72^3, 800 bands 1046 -> 856.
+template <typename T> void x_tile(const qgb_sphere& s, int nb, int* nc, int* threads) {
+  const int cols = s.N[1] * s.N[2], L1 = s.L1[0], L2 = s.L2[0];
   double best = 1e30;
-  for (int z = 1; z <= 8; ++z) {
-    const int nz = (N2 + z - 1) / z;
-    const size_t smem = x_smem_bytes(s, nz, 16);
-    if ((nz < 16 && z > 1) || smem > kSmemPerSm) continue;
-    double c;
-    const int t = pick_threads(nz * s.L1[0], nz * s.L2[0], smem, kThreads, &c);
-    c *= z;                           // parts per row
-    c += 0.5 * z * s.N[0];            // tables of each CTA
-    if (c < best) {
-      best = c;
-      *zs = z;
-      *threads = t;
+  *nc = std::min(cols, 32);
+  *threads = 128;
+  for (int c = 32; c <= 256; c += 16) {
+    const size_t smem = x_smem_bytes(s, c, sizeof(cplx_t<T>));
+    if (c > 32 && (smem > kSmemPerSm || c >= cols + 16)) break;
+    for (int t = 64; t <= kThreads; t += 32) {
+      const int outer = L2 > 1 ? (c * L1 + t - 1) / t : 0, mid = (c * L2 + t - 1) / t;
+      const double work = 2.0 * (outer * L2 + mid * L1) + 8.0 + 4.0 * s.N[0] / t;
+      const double cost = launch_cost<T>(static_cast<double>((cols + c - 1) / c) * nb * s.nk, t, smem, work);
+      if (cost < best * 0.999) {
+        best = cost;
+        *nc = std::min(c, cols);
+        *threads = t;
+      }
     }
   }
 }
@@ -668,7 +682,7 @@ template <typename T>
 int launch_ifft_yz(const qgb_sphere& s, const LocalParams& lp, const void* C, void* planes, cudaStream_t st) {
   const size_t smem = yz_smem_bytes(s, sizeof(cplx_t<T>));
   if (int rc = raise_smem_limit(k_ifft_yz<T>, smem)) return rc;
-  k_ifft_yz<T><<<dim3(s.max_slabs, lp.nb, s.nk), threads_yz<T>(s), smem, st>>>(
+  k_ifft_yz<T><<<dim3(s.max_slabs, lp.nb, s.nk), threads_yz<T>(s, lp.nb), smem, st>>>(
       s, lp, static_cast<const cplx_t<T>*>(C), static_cast<cplx_t<T>*>(planes));
   QGB_LAUNCH_CHECK("k_ifft_yz");
   return QGB_OK;
@@ -680,17 +694,16 @@ int launch_chunk(const qgb_sphere& s, const LocalParams& lp, const void* C, void
   using C2 = cplx_t<T>;
   int rc;
   if ((rc = launch_ifft_yz<T>(s, lp, C, planes, st))) return rc;
-  int zs, tx;
-  x_split<T>(s, &zs, &tx);
-  const int nzp = (s.N[2] + zs - 1) / zs;
-  const size_t smx = x_smem_bytes(s, nzp, sizeof(C2));
+  int nc, tx;
+  x_tile<T>(s, lp.nb, &nc, &tx);
+  const size_t smx = x_smem_bytes(s, nc, sizeof(C2));
   if ((rc = raise_smem_limit(k_xpass<T>, smx))) return rc;
-  k_xpass<T><<<dim3(s.N[1] * zs, lp.nb, s.nk), tx, smx, st>>>(s, lp, static_cast<C2*>(planes), zs, nzp);
+  k_xpass<T><<<dim3((s.N[1] * s.N[2] + nc - 1) / nc, lp.nb, s.nk), tx, smx, st>>>(s, lp, static_cast<C2*>(planes), nc);
   QGB_LAUNCH_CHECK("k_xpass");
   if (gather_after) QGB_CUDA_CHECK(cudaStreamWaitEvent(st, gather_after, 0));
   const size_t smem = yz_smem_bytes(s, sizeof(C2));
   if ((rc = raise_smem_limit(k_fft_yz_gather<T>, smem))) return rc;
-  k_fft_yz_gather<T><<<dim3(s.max_slabs, lp.nb, s.nk), threads_yz<T>(s), smem, st>>>(
+  k_fft_yz_gather<T><<<dim3(s.max_slabs, lp.nb, s.nk), threads_yz<T>(s, lp.nb), smem, st>>>(
       s, lp, static_cast<const C2*>(C), static_cast<C2*>(out), static_cast<const C2*>(planes));
   QGB_LAUNCH_CHECK("k_fft_yz_gather");
   return QGB_OK;
