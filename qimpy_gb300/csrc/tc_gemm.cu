@@ -3,16 +3,29 @@
 // D[m][n] = sum_k A[m][k] B[n][k] (both operands K-major, "TN") is computed as
 //   A_hi B_hi^T + A_hi B_lo^T + A_lo B_hi^T,   x_hi = bf16(x), x_lo = bf16(x - x_hi),
 // with FP32 accumulation in tensor memory: about 16 significant bits per
-// product, the split-BF16x3 scheme.  The three products run as one K loop
-// over three segments, so a CTA accumulates them into one TMEM tile.
+// product, the split-BF16x3 scheme.  How the three products meet (Order):
+//   ORDER_SEGMENTS  one after the other over the whole K range, into one
+//                   accumulator (the subspace overlaps, whose FP64 results keep
+//                   their bits);
+//   ORDER_BLOCKS    the three of a K block together, so a block takes 4 operand
+//                   tiles from L2 and not 6;
+//   ORDER_SPLIT     the same with the two small products in an accumulator of
+//                   their own, added at the end: a third of the roundings at
+//                   the size of the result, for long K ranges.
 //
-// Per CTA (128 threads, one 128 x BN output tile, one K range):
-//   thread 0 (warp 0)  - TMA producer: 128B-swizzled A and B boxes into an
-//                        S-stage shared-memory ring, mbarrier complete_tx;
-//   thread 32 (warp 1) - MMA issuer: tcgen05.mma.cta_group::1.kind::f16 with
-//                        bf16 inputs and an FP32 accumulator in TMEM, four K=16
-//                        steps per 64-wide stage, tcgen05.commit frees the stage;
-//   all 4 warps        - epilogue: tcgen05.ld of their 32 TMEM lanes.
+// Persistent CTAs, one per SM (192 threads); a unit is a 128 x BN output tile of
+// one K range, N tiles fastest:
+//   warps 0-3 - epilogue: tcgen05.ld of their 32 TMEM lanes, from one of two
+//               accumulators (256 columns each) while the next unit's MMAs fill
+//               the other;
+//   warp 4    - TMA producer: 128B-swizzled boxes of A_hi, A_lo, B_hi and B_lo of
+//               a K = 64 block into one stage of a shared-memory ring, so the
+//               three products take 4 tiles from L2 and not 6 (the SM's ingest,
+//               64 B a cycle, is the bound: 96 KB and 1536 MMA cycles per block
+//               at BN = 256);
+//   warp 5    - MMA issuer: tcgen05.mma.cta_group::1.kind::f16 with bf16 inputs
+//               and an FP32 accumulator, twelve K = 16 steps per stage.
+// BN is the smallest multiple of 32 that covers the band rows in equal tiles.
 // Every mbarrier wait is bounded by a %globaltimer deadline; on timeout the
 // kernel records an error code, drains its own TMA copies (bounded), frees its
 // TMEM and returns.
@@ -22,6 +35,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "tcgen05.cuh"
 
@@ -30,12 +44,20 @@ namespace tc {
 
 constexpr int BM = 128;            // MMA M (rows of A per CTA)
 constexpr int BK = 64;             // bf16 elements per stage along K (one 128 B swizzle atom)
-constexpr int kThreads = 128;
+constexpr int EPI_WARPS = 4;
+constexpr int kThreads = (EPI_WARPS + 2) * 32;
+constexpr int kSms = 152;
+constexpr int ACC_COLS = 256;      // TMEM columns of one accumulator (two of them)
+constexpr int MAX_STAGES = 4;
 
 enum Epi { EPI_PARTIAL = 0, EPI_ADD_HC = 1 };
+enum Order { ORDER_SEGMENTS = 0, ORDER_BLOCKS = 1, ORDER_SPLIT = 2 };
 
 struct GemmArgs {
   int M, N, K;             // logical sizes (rows of A, rows of B, reduction)
+  int BN, HB, stages;      // tile width (rows of B), bands per tile, ring depth
+  int order;
+  int units, m_tiles, n_tiles;
   int kb_per_split;        // 64-wide K blocks per split
   int splits;
   float* partial;          // EPI_PARTIAL: [batch][split][m_tiles*BM][n_tiles*BN]
@@ -50,155 +72,226 @@ struct GemmArgs {
   int skip_loads;          // test aid: the producer issues no copies, so the MMA wait runs out
 };
 
-template <int BN, int STAGES>
-struct Smem {
-  static constexpr int A_BYTES = BM * BK * 2;   // 16 KB
-  static constexpr int B_BYTES = BN * BK * 2;   // BN x 128 B
-  static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-  static constexpr int BAR_OFF = STAGES * STAGE_BYTES;
-  static constexpr int TOTAL = BAR_OFF + (2 * STAGES + 1) * 8 + 16 + 1024;  // + alignment slack
-};
+constexpr int A_BYTES = BM * BK * 2;  // one of A_hi, A_lo: 16 KB
+__host__ __device__ constexpr int stage_bytes(int bn, int order) {
+  return (A_BYTES + bn * BK * 2) * (order == ORDER_SEGMENTS ? 1 : 2);
+}
+constexpr int BAR_BYTES = (2 * MAX_STAGES + 5) * 8 + 16;
+__host__ __device__ constexpr int smem_bytes(int bn, int order, int stages) {
+  return stages * stage_bytes(bn, order) + BAR_BYTES + 1024;  // + alignment slack
+}
 
-template <int BN, int STAGES, int EPI>
-__global__ void __launch_bounds__(kThreads)
+struct Unit {
+  int n_tile, m_tile, split, batch;
+};
+__device__ __forceinline__ Unit unit_of(const GemmArgs& a, int u) {
+  Unit t;
+  t.n_tile = u % a.n_tiles;
+  u /= a.n_tiles;
+  t.m_tile = u % a.m_tiles;
+  u /= a.m_tiles;
+  t.split = u % a.splits;
+  t.batch = u / a.splits;
+  return t;
+}
+
+template <int EPI>
+__global__ void __launch_bounds__(kThreads, 1)
     k_tc_gemm(const __grid_constant__ CUtensorMap mA_hi, const __grid_constant__ CUtensorMap mA_lo,
               const __grid_constant__ CUtensorMap mB_hi, const __grid_constant__ CUtensorMap mB_lo,
               const GemmArgs args) {
-  using L = Smem<BN, STAGES>;
   extern __shared__ __align__(1024) unsigned char tc_smem_raw[];
   // 1024-byte alignment for the 128B-swizzled tiles.
   unsigned char* smem = reinterpret_cast<unsigned char*>(
       (reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
-  uint64_t* empty = full + STAGES;
-  uint64_t* tmem_full = empty + STAGES;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_full + 1);
+  const int BN = args.BN, S = args.stages, STAGE = stage_bytes(BN, args.order), B_BYTES = BN * BK * 2;
+  const int segments = args.order == ORDER_SEGMENTS ? 3 : 1;
+  // Accumulators: two in turn, or (ORDER_SPLIT) the products' own two.
+  const int bufs = args.order == ORDER_SPLIT ? 1 : 2;
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + S * STAGE);
+  uint64_t* empty = full + MAX_STAGES;
+  uint64_t* acc_full = empty + MAX_STAGES;  // [2]
+  uint64_t* acc_empty = acc_full + 2;       // [2]
+  uint64_t* done = acc_empty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int m_tile = blockIdx.x, n_tile = blockIdx.y;
-  const int batch = blockIdx.z / args.splits, split = blockIdx.z % args.splits;
   const int nkb_total = (args.K + BK - 1) / BK;
-  const int kb0 = split * args.kb_per_split;
-  const int kb1 = min(nkb_total, kb0 + args.kb_per_split);
-  const int nkb = max(0, kb1 - kb0);
-  const int niter = 3 * nkb;  // segments: (hi, hi), (hi, lo), (lo, hi)
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < S; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
-    mbar_init(tmem_full, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&acc_full[i], 1);
+      mbar_init(&acc_empty[i], EPI_WARPS);
+    }
+    mbar_init(done, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) tmem_alloc(tmem_slot, BN);
+  if (warp == EPI_WARPS + 1) tmem_alloc(tmem_slot, 2 * ACC_COLS);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  if (threadIdx.x == 0 && niter > 0 && !args.skip_loads) {
+  if (threadIdx.x == EPI_WARPS * 32 && !args.skip_loads) {
     // ---------------- TMA producer ----------------
-    int issued = 0;
-    for (int it = 0; it < niter; ++it) {
-      const int s = it % STAGES, use = it / STAGES;
-      if (use > 0 && !mbar_wait(&empty[s], (use - 1) & 1, args.err, 1, args.timeout_ns)) break;
-      const int seg = it / nkb, kb = kb0 + it % nkb;
-      unsigned char* a_dst = smem + s * L::STAGE_BYTES;
-      unsigned char* b_dst = a_dst + L::A_BYTES;
-      mbar_arrive_expect_tx(&full[s], L::STAGE_BYTES);
-      tma_load_3d(a_dst, seg == 2 ? &mA_lo : &mA_hi, &full[s], kb * BK, m_tile * BM, batch);
-      tma_load_3d(b_dst, seg == 1 ? &mB_lo : &mB_hi, &full[s], kb * BK, n_tile * BN, batch);
-      ++issued;
+    int it = 0;  // stages filled so far, over all units
+    bool live = true;
+    for (int u = blockIdx.x; u < args.units && live; u += gridDim.x) {
+      const Unit t = unit_of(args, u);
+      const int kb0 = t.split * args.kb_per_split, nkb = min(nkb_total, kb0 + args.kb_per_split) - kb0;
+      for (int i = 0; i < segments * nkb; ++i, ++it) {
+        const int s = it % S, use = it / S;
+        if (use > 0 && !mbar_wait(&empty[s], (use - 1) & 1, args.err, 1, args.timeout_ns)) {
+          live = false;
+          break;
+        }
+        const int seg = i / nkb, k = (kb0 + i - seg * nkb) * BK;
+        unsigned char* dst = smem + s * STAGE;
+        mbar_arrive_expect_tx(&full[s], STAGE);
+        if (segments == 3) {
+          tma_load_3d(dst, seg == 2 ? &mA_lo : &mA_hi, &full[s], k, t.m_tile * BM, t.batch);
+          tma_load_3d(dst + A_BYTES, seg == 1 ? &mB_lo : &mB_hi, &full[s], k, t.n_tile * BN, t.batch);
+        } else {
+          tma_load_3d(dst, &mA_hi, &full[s], k, t.m_tile * BM, t.batch);
+          tma_load_3d(dst + 2 * A_BYTES, &mB_hi, &full[s], k, t.n_tile * BN, t.batch);
+          tma_load_3d(dst + 2 * A_BYTES + B_BYTES, &mB_lo, &full[s], k, t.n_tile * BN, t.batch);
+          tma_load_3d(dst + A_BYTES, &mA_lo, &full[s], k, t.m_tile * BM, t.batch);
+        }
+      }
     }
-    // Drain: every load issued lands before exit.  Loads before the last
-    // STAGES were waited for through the empty barriers (their MMAs consumed
-    // them); the last min(STAGES, issued) are waited for here, even after an
-    // error.
-    for (int it = max(0, issued - STAGES); it < issued; ++it)
-      mbar_drain(&full[it % STAGES], (it / STAGES) & 1, args.err, 2);
-  } else if (threadIdx.x == 32 && niter > 0) {
+    // Drain: every load issued lands before exit.  Loads before the last S were
+    // waited for through the empty barriers (their MMAs consumed them); the
+    // last min(S, issued) are waited for here, even after an error.
+    for (int i = max(0, it - S); i < it; ++i) mbar_drain(&full[i % S], (i / S) & 1, args.err, 2);
+  } else if (threadIdx.x == (EPI_WARPS + 1) * 32) {
     // ---------------- MMA issuer ----------------
-    constexpr uint32_t idesc = idesc_bf16_f32(BM, BN);
-    for (int it = 0; it < niter; ++it) {
-      const int s = it % STAGES, use = it / STAGES;
-      if (!mbar_wait(&full[s], use & 1, args.err, 3, args.timeout_ns)) break;
+    const uint32_t idesc = idesc_bf16_f32(BM, BN);
+    const uint32_t b_step = static_cast<uint32_t>(B_BYTES / 16);
+    int it = 0, n = 0;  // stages and units so far
+    bool live = true;
+    for (int u = blockIdx.x; u < args.units && live; u += gridDim.x, ++n) {
+      const Unit t = unit_of(args, u);
+      const int kb0 = t.split * args.kb_per_split, nkb = min(nkb_total, kb0 + args.kb_per_split) - kb0;
+      const int buf = n % bufs;
+      const uint32_t acc = tmem + buf * ACC_COLS, acc2 = bufs == 1 ? tmem + ACC_COLS : acc;
+      if (n >= bufs && !mbar_wait(&acc_empty[buf], (n / bufs - 1) & 1, args.err, 5, args.timeout_ns)) break;
       tc_fence_after();
-      const uint32_t a_addr = smem_u32(smem + s * L::STAGE_BYTES);
-      const uint32_t b_addr = a_addr + L::A_BYTES;
-      const uint64_t adesc = desc_kmajor_sw128(a_addr), bdesc = desc_kmajor_sw128(b_addr);
+      for (int i = 0; i < segments * nkb; ++i, ++it) {
+        const int s = it % S;
+        if (!mbar_wait(&full[s], (it / S) & 1, args.err, 3, args.timeout_ns)) {
+          live = false;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t addr = smem_u32(smem + s * STAGE);
+        const uint64_t a_hi = desc_kmajor_sw128(addr);
+        const uint64_t b_hi = desc_kmajor_sw128(addr + (segments == 3 ? A_BYTES : 2 * A_BYTES));
 #pragma unroll
-      for (int k = 0; k < BK / 16; ++k)  // K = 16 per MMA: advance 32 B = 2 descriptor units
-        umma_bf16(tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (it > 0 || k > 0) ? 1u : 0u);
-      umma_commit(&empty[s]);
+        for (int k = 0; k < BK / 16; ++k)  // K = 16 per MMA: advance 32 B = 2 descriptor units
+          umma_bf16(acc, a_hi + 2 * k, b_hi + 2 * k, idesc, (i > 0 || k > 0) ? 1u : 0u);
+        if (segments == 1) {
+          const uint64_t a_lo = a_hi + A_BYTES / 16, b_lo = b_hi + b_step;
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k)
+            umma_bf16(acc2, a_hi + 2 * k, b_lo + 2 * k, idesc, (bufs == 1 && i == 0 && k == 0) ? 0u : 1u);
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k) umma_bf16(acc2, a_lo + 2 * k, b_hi + 2 * k, idesc, 1u);
+        }
+        umma_commit(&empty[s]);
+      }
+      umma_commit(&acc_full[buf]);
     }
-    umma_commit(tmem_full);  // fires once every MMA issued above has completed
+    umma_commit(done);  // fires once every MMA issued above has completed
+  } else if (warp < EPI_WARPS) {
+    // ---------------- Epilogue ----------------
+    int n = 0;
+    for (int u = blockIdx.x; u < args.units; u += gridDim.x, ++n) {
+      const Unit t = unit_of(args, u);
+      const int buf = n % bufs;
+      bool ok = mbar_wait(&acc_full[buf], (n / bufs) & 1, args.err, 4, 2 * kTimeoutNs);
+      // tcgen05.ld is warp-collective: decide per warp.
+      ok = __all_sync(0xffffffffu, ok && *reinterpret_cast<volatile int*>(args.err) == 0);
+      if (!ok) break;
+      tc_fence_after();
+      const bool any = t.split * args.kb_per_split < nkb_total;  // an empty K range adds nothing
+      const int row = t.m_tile * BM + warp * 32 + lane;
+      const uint32_t trow = tmem + buf * ACC_COLS + (static_cast<uint32_t>(warp * 32) << 16);
+      if (EPI == EPI_PARTIAL) {
+        float* out = args.partial + ((static_cast<long long>(t.batch) * args.splits + t.split) * args.part_rows + row) *
+                                        args.part_ld + t.n_tile * BN;
+#pragma unroll 1
+        for (int c0 = 0; c0 < BN; c0 += 32) {
+          float v[32];
+          tmem_ld32(trow + c0, v);
+          if (bufs == 1) {
+            float w[32];
+            tmem_ld32(trow + ACC_COLS + c0, w);
+#pragma unroll
+            for (int i = 0; i < 32; ++i) v[i] += w[i];
+          }
+#pragma unroll
+          for (int i = 0; i < 32; i += 4)
+            *reinterpret_cast<float4*>(out + c0 + i) =
+                any ? make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+      } else {
+        // Columns [0, HB) hold real parts and [HB, BN) imaginary parts of bands
+        // n_tile * HB + j; rows are basis entries g.
+        const int HB = args.HB;
+        const bool row_ok = row < args.M;
+        float2* hc = args.hc + t.batch * args.hc_batch_stride + row;
+#pragma unroll 1
+        for (int c0 = 0; c0 < HB; c0 += 16) {
+          float vr[16], vi[16];
+          // All loads of HC first, then the stores: interleaved read-modify-
+          // writes through one pointer could alias, which would serialise the
+          // memory round trips.
+          float2 o[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) {
+            const int b = t.n_tile * HB + c0 + i;
+            o[i] = (!args.hc_store && row_ok && b < args.nb) ? hc[static_cast<long long>(b) * args.hc_ld]
+                                                             : make_float2(0.f, 0.f);
+          }
+          tmem_ld16(trow + c0, vr);
+          tmem_ld16(trow + HB + c0, vi);
+          if (bufs == 1) {
+            float wr[16], wi[16];
+            tmem_ld16(trow + ACC_COLS + c0, wr);
+            tmem_ld16(trow + ACC_COLS + HB + c0, wi);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              vr[i] += wr[i];
+              vi[i] += wi[i];
+            }
+          }
+          if (row_ok) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) {
+              const int b = t.n_tile * HB + c0 + i;
+              if (b < args.nb)
+                hc[static_cast<long long>(b) * args.hc_ld] = make_float2(o[i].x + vr[i], o[i].y + vi[i]);
+            }
+          }
+        }
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&acc_empty[buf]);
+    }
+    // Every MMA issued has completed before TMEM is freed, error or not.
+    mbar_drain(done, 0, args.err, 6);
+    tc_fence_before();
   }
   __syncwarp();
-
-  // ---------------- Epilogue: all four warps ----------------
-  // tmem_full is committed after every MMA the issuer launched (also when it
-  // stopped early), so this wait drains the tensor cores before TMEM is read
-  // or freed, error or not.
-  bool ok = niter > 0;
-  if (ok) ok = mbar_drain(tmem_full, 0, args.err, 4);
-  tc_fence_after();
-  // tcgen05.ld is warp-collective: decide per warp.
-  ok = __all_sync(0xffffffffu, ok && *reinterpret_cast<volatile int*>(args.err) == 0);
-  if (ok) {
-    const int row = m_tile * BM + warp * 32 + lane;
-    const uint32_t trow = tmem + (static_cast<uint32_t>(warp * 32) << 16);
-    if (EPI == EPI_PARTIAL) {
-      float* out = args.partial + ((static_cast<long long>(batch) * args.splits + split) * args.part_rows + row) *
-                                      args.part_ld + n_tile * BN;
-#pragma unroll 1
-      for (int c0 = 0; c0 < BN; c0 += 32) {
-        float v[32];
-        tmem_ld32(trow + c0, v);
-#pragma unroll
-        for (int i = 0; i < 32; i += 4)
-          *reinterpret_cast<float4*>(out + c0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-      }
-    } else {
-      // Columns [0, BN/2) hold real parts and [BN/2, BN) imaginary parts of
-      // bands n_tile*BN/2 + j; rows are basis entries g.
-      constexpr int HB = BN / 2;
-      const bool row_ok = row < args.M;
-      float2* hc = args.hc + batch * args.hc_batch_stride + row;
-#pragma unroll 1
-      for (int c0 = 0; c0 < HB; c0 += 32) {
-        float vr[32], vi[32];
-        // All 32 loads of HC first, then the stores: interleaved read-modify-
-        // writes through one pointer could alias, which would serialise 32
-        // memory round trips per thread.
-        float2 o[32];
-        if (args.hc_store) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = make_float2(0.f, 0.f);
-        } else if (row_ok) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int b = n_tile * HB + c0 + i;
-            o[i] = b < args.nb ? hc[static_cast<long long>(b) * args.hc_ld] : make_float2(0.f, 0.f);
-          }
-        }
-        tmem_ld32(trow + c0, vr);
-        tmem_ld32(trow + HB + c0, vi);
-        if (row_ok) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int b = n_tile * HB + c0 + i;
-            if (b < args.nb) hc[static_cast<long long>(b) * args.hc_ld] = make_float2(o[i].x + vr[i], o[i].y + vi[i]);
-          }
-        }
-      }
-    }
-  }
-  tc_fence_before();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == EPI_WARPS + 1) {
     tc_fence_after();
-    tmem_dealloc(tmem, BN);
+    tmem_dealloc(tmem, 2 * ACC_COLS);
   }
 }
 
@@ -233,23 +326,53 @@ struct Operand {
   long long rows, ld, batch_stride;
 };
 
-template <int BN, int STAGES, int EPI>
-static int launch(const Operand& A, const Operand& B, int K, int batch, const GemmArgs& args_in,
-                  cudaStream_t st) {
-  using L = Smem<BN, STAGES>;
-  GemmArgs base_args = args_in;
-  if (base_args.timeout_ns == 0) base_args.timeout_ns = kTimeoutNs;
+// Tile of `nb` bands: rows of B per tile (real and imaginary rows of HB bands
+// each, HB a multiple of 16), as few tiles as 256 rows allow and those equal.
+static int band_tile(int nb) {
+  const int tiles = (nb + 127) / 128, hb = (nb + tiles - 1) / tiles;
+  return 2 * std::max(16, (hb + 15) / 16 * 16);
+}
+static int ring_depth(int bn, int order) {
+  return std::min(MAX_STAGES, (227 * 1024 - BAR_BYTES - 1024) / stage_bytes(bn, order));
+}
+
+// K splits of a product of `tiles` output tiles of 128 x bn and nkb K blocks: the
+// number that needs the least time, a block taking its copies' 64 B a cycle, a
+// unit some 2000 cycles more, a split the write and read of its partial sums.
+static int pick_splits(int tiles, int nkb, int bn) {
+  int best = 1;
+  double best_cost = 1e30;
+  for (int s = 1; s <= std::min(nkb, 64); ++s) {
+    const int per = (nkb + s - 1) / s;
+    const double waves = std::ceil(static_cast<double>(tiles) * ((nkb + per - 1) / per) / kSms);
+    const double cost = waves * (per * (stage_bytes(bn, ORDER_SPLIT) / 64.0) + 2000.0) +
+                        static_cast<double>(tiles) * s * (BM * bn * 8.0) / 2500.0;
+    if (cost < best_cost * 0.999) {
+      best_cost = cost;
+      best = s;
+    }
+  }
+  return best;
+}
+
+template <int EPI>
+static int launch(const Operand& A, const Operand& B, int K, int batch, const GemmArgs& args_in, cudaStream_t st) {
+  GemmArgs args = args_in;
+  if (args.timeout_ns == 0) args.timeout_ns = kTimeoutNs;
   CUtensorMap ma_hi, ma_lo, mb_hi, mb_lo;
   int rc;
   if ((rc = make_map(&ma_hi, A.hi, K, A.rows, batch, A.ld, A.batch_stride, BM))) return rc;
   if ((rc = make_map(&ma_lo, A.lo, K, A.rows, batch, A.ld, A.batch_stride, BM))) return rc;
-  if ((rc = make_map(&mb_hi, B.hi, K, B.rows, batch, B.ld, B.batch_stride, BN))) return rc;
-  if ((rc = make_map(&mb_lo, B.lo, K, B.rows, batch, B.ld, B.batch_stride, BN))) return rc;
-  if ((rc = raise_smem_limit(k_tc_gemm<BN, STAGES, EPI>, L::TOTAL))) return rc;
-  const int m_tiles = static_cast<int>((A.rows + BM - 1) / BM);
-  const int n_tiles = static_cast<int>((B.rows + BN - 1) / BN);
-  dim3 grid(m_tiles, n_tiles, batch * base_args.splits);
-  k_tc_gemm<BN, STAGES, EPI><<<grid, kThreads, L::TOTAL, st>>>(ma_hi, ma_lo, mb_hi, mb_lo, base_args);
+  if ((rc = make_map(&mb_hi, B.hi, K, B.rows, batch, B.ld, B.batch_stride, args.BN))) return rc;
+  if ((rc = make_map(&mb_lo, B.lo, K, B.rows, batch, B.ld, B.batch_stride, args.BN))) return rc;
+  args.HB = args.BN / 2;
+  args.stages = ring_depth(args.BN, args.order);
+  const size_t smem = smem_bytes(args.BN, args.order, args.stages);
+  if ((rc = raise_smem_limit(k_tc_gemm<EPI>, smem))) return rc;
+  args.m_tiles = static_cast<int>((A.rows + BM - 1) / BM);
+  args.n_tiles = static_cast<int>((B.rows + args.BN - 1) / args.BN);
+  args.units = args.m_tiles * args.n_tiles * batch * args.splits;
+  k_tc_gemm<EPI><<<std::min(args.units, kSms), kThreads, smem, st>>>(ma_hi, ma_lo, mb_hi, mb_lo, args);
   QGB_LAUNCH_CHECK("k_tc_gemm");
   return QGB_OK;
 }
@@ -263,36 +386,71 @@ __device__ __forceinline__ void split_bf16(float x, __nv_bfloat16& hi, __nv_bflo
   lo = __float2bfloat16_rn(x - __bfloat162float(hi));
 }
 
-// Wavefunction rows for the B operand: complex64 C[k][nb][n_tot] -> rows
-// r = t*BN + part*HB + j (band t*HB + j, part 0 = real, 1 = imaginary) of
-// [k][rows][ld] bf16 hi/lo; bands >= nb give zero rows.  With `weight`
-// (real wavefunctions: 1 on the Gz = 0 plane, 2 elsewhere; powers of two, so
-// the split stays exact) every coefficient is scaled by w_g.
-__global__ void k_split_bands(const float2* __restrict__ C, int nb, int n_tot, int HB, int rows, int ld,
-                              const double* __restrict__ weight, __nv_bfloat16* __restrict__ hi,
-                              __nv_bfloat16* __restrict__ lo) {
-  const int r = blockIdx.y, k = blockIdx.z;
-  const int t = r / (2 * HB), rem = r - t * 2 * HB, part = rem / HB, b = t * HB + rem % HB;
+__device__ __forceinline__ unsigned pack_pair(__nv_bfloat16 a, __nv_bfloat16 b) {
+  return static_cast<unsigned>(__bfloat16_as_ushort(a)) | (static_cast<unsigned>(__bfloat16_as_ushort(b)) << 16);
+}
+// 4 values -> their bf16 hi and lo parts, 8 B each.
+__device__ __forceinline__ void split4(const float (&v)[4], uint2& hi, uint2& lo) {
+  __nv_bfloat16 h[4], l[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) split_bf16(v[i], h[i], l[i]);
+  hi = make_uint2(pack_pair(h[0], h[1]), pack_pair(h[2], h[3]));
+  lo = make_uint2(pack_pair(l[0], l[1]), pack_pair(l[2], l[3]));
+}
+
+// Bands as operand rows: complex64 C[k][nb][n_tot] -> rows r = t*2HB + part*HB + j
+// (band t*HB + j, part 0 = real, 1 = imaginary) of [k][rows][ld] bf16 hi/lo;
+// bands >= nb give zero rows.  With `weight` (real wavefunctions: 1 on the
+// Gz = 0 plane, 2 elsewhere; powers of two, so the split stays exact) every
+// coefficient is scaled by w_g.  A thread takes 4 basis entries of a band, both
+// parts: bound by its 16 B moved per entry (one part and one entry a thread,
+// reading everything twice: 107 us against 51 for 4 x 200 x 19926).
+__global__ void __launch_bounds__(256) k_split_bands(const float2* __restrict__ C, int nb, int n_tot, int HB, int rows,
+                                                     int ld, const double* __restrict__ weight,
+                                                     __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo) {
+  const int b = blockIdx.y, k = blockIdx.z;
+  const int t = b / HB, r = t * 2 * HB + (b - t * HB);
   const float2* src = C + (static_cast<long long>(k) * nb + b) * n_tot;
-  const long long o = (static_cast<long long>(k) * rows + r) * ld;
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ld; g += gridDim.x * blockDim.x) {
-    float v = 0.f;
-    if (b < nb && g < n_tot) {
-      const float2 c = src[g];
-      v = part ? c.y : c.x;
-      if (weight) v *= static_cast<float>(weight[g]);
+  const long long o_re = (static_cast<long long>(k) * rows + r) * ld, o_im = o_re + static_cast<long long>(HB) * ld;
+  for (int g = 4 * (blockIdx.x * blockDim.x + threadIdx.x); g < ld; g += 4 * gridDim.x * blockDim.x) {
+    float re[4], im[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float2 c = make_float2(0.f, 0.f);
+      if (b < nb && g + i < n_tot) {
+        c = src[g + i];
+        if (weight) {
+          const float w = static_cast<float>(weight[g + i]);
+          c.x *= w;
+          c.y *= w;
+        }
+      }
+      re[i] = c.x;
+      im[i] = c.y;
     }
-    __nv_bfloat16 h, l;
-    split_bf16(v, h, l);
-    hi[o + g] = h;
-    lo[o + g] = l;
+    uint2 h, l;
+    split4(re, h, l);
+    *reinterpret_cast<uint2*>(hi + o_re + g) = h;
+    *reinterpret_cast<uint2*>(lo + o_re + g) = l;
+    split4(im, h, l);
+    *reinterpret_cast<uint2*>(hi + o_im + g) = h;
+    *reinterpret_cast<uint2*>(lo + o_im + g) = l;
   }
+}
+
+static int launch_split_bands(const void* C, int nb, int nk, int n_tot, int HB, long long rows, long long ld,
+                              const double* weight, __nv_bfloat16* hi, __nv_bfloat16* lo, cudaStream_t st) {
+  const dim3 grid(static_cast<unsigned>(std::min<long long>(32, (ld + 1023) / 1024)), static_cast<unsigned>(rows / 2), nk);
+  k_split_bands<<<grid, 256, 0, st>>>(static_cast<const float2*>(C), nb, n_tot, HB, static_cast<int>(rows),
+                                      static_cast<int>(ld), weight, hi, lo);
+  QGB_LAUNCH_CHECK("k_split_bands");
+  return QGB_OK;
 }
 
 // Projector operands, once per basis: complex64 beta[k][P][n_tot] ->
 //   A  [k][2P][ldA]  rows (Re beta_p; Im beta_p), K = basis  (for <beta|psi>)
 //   AT [k][n_tot][ldT] row g = (Re beta_p(g), p < P; Im beta_p(g)), K = 2P
-//                                                     (for beta (D proj); skipped when t_hi is NULL)
+//                                                     (for beta (D proj))
 __global__ void k_split_beta(const float2* __restrict__ beta, int P, int n_tot, int ldA, int ldT,
                              __nv_bfloat16* __restrict__ a_hi, __nv_bfloat16* __restrict__ a_lo,
                              __nv_bfloat16* __restrict__ t_hi, __nv_bfloat16* __restrict__ t_lo) {
@@ -306,7 +464,7 @@ __global__ void k_split_beta(const float2* __restrict__ beta, int P, int n_tot, 
     split_bf16(c.x, h, l);
     a_hi[oa_r + g] = h;
     a_lo[oa_r + g] = l;
-    if (t_hi != nullptr && g < n_tot) {
+    if (g < n_tot) {
       const long long ot = (static_cast<long long>(k) * n_tot + g) * ldT;
       t_hi[ot + p] = h;
       t_lo[ot + p] = l;
@@ -314,7 +472,7 @@ __global__ void k_split_beta(const float2* __restrict__ beta, int P, int n_tot, 
     split_bf16(c.y, h, l);
     a_hi[oa_i + g] = h;
     a_lo[oa_i + g] = l;
-    if (t_hi != nullptr && g < n_tot) {
+    if (g < n_tot) {
       const long long ot = (static_cast<long long>(k) * n_tot + g) * ldT;
       t_hi[ot + P + p] = h;
       t_lo[ot + P + p] = l;
@@ -384,16 +542,16 @@ __global__ void k_reduce_gram(const float* __restrict__ partial, int splits, lon
 }
 
 // Dp[b][p] = sum_q D_atom[a][p'][q'] projT[b][a*pa + q'] (block-diagonal D),
-// written as the back-projection B operand: rows r = t*BN + part*HB + j for
+// written as the back-projection B operand: rows r = t*2HB + part*HB + j for
 // band t*HB + j, K = 2P: real-output row (Re Dp, -Im Dp), imaginary-output
-// row (Im Dp, Re Dp).
+// row (Im Dp, Re Dp).  One CTA per band computes both rows.
 __global__ void k_dapply_split(const float2* __restrict__ projT, const float2* __restrict__ D, int n_atoms,
                                int pa, int nb, int HB, int rows, int ld, __nv_bfloat16* __restrict__ hi,
                                __nv_bfloat16* __restrict__ lo) {
   const int P = n_atoms * pa;
-  const int r = blockIdx.y, k = blockIdx.z;
-  const int t = r / (2 * HB), rem = r - t * 2 * HB, part = rem / HB, b = t * HB + rem % HB;
-  const long long o = (static_cast<long long>(k) * rows + r) * ld;
+  const int b = blockIdx.y, k = blockIdx.z;
+  const int t = b / HB, r = t * 2 * HB + (b - t * HB);
+  const long long o_re = (static_cast<long long>(k) * rows + r) * ld, o_im = o_re + static_cast<long long>(HB) * ld;
   for (int p = threadIdx.x; p < ld; p += blockDim.x) {
     float re = 0.f, im = 0.f;
     if (b < nb && p < P) {
@@ -408,63 +566,75 @@ __global__ void k_dapply_split(const float2* __restrict__ projT, const float2* _
     }
     __nv_bfloat16 h, l;
     if (p < P) {
-      split_bf16(part ? im : re, h, l);
-      hi[o + p] = h;
-      lo[o + p] = l;
-      split_bf16(part ? re : -im, h, l);
-      hi[o + P + p] = h;
-      lo[o + P + p] = l;
+      split_bf16(re, h, l);
+      hi[o_re + p] = hi[o_im + P + p] = h;
+      lo[o_re + p] = lo[o_im + P + p] = l;
+      split_bf16(im, h, l);
+      hi[o_im + p] = h;
+      lo[o_im + p] = l;
+      hi[o_re + P + p] = __hneg(h);
+      lo[o_re + P + p] = __hneg(l);
     } else if (p >= 2 * P) {
-      hi[o + p] = __float2bfloat16_rn(0.f);
-      lo[o + p] = __float2bfloat16_rn(0.f);
+      const __nv_bfloat16 z = __float2bfloat16_rn(0.f);
+      hi[o_re + p] = lo[o_re + p] = hi[o_im + p] = lo[o_im + p] = z;
     }
   }
 }
 
 // Band rotation operands.  C complex64 [k][n_in][n] -> A [k][n][ldA]: row g =
-// (Re C_i(g), i < n_in; Im C_i(g)), K = 2 n_in, through a 32 x 32 shared tile
-// (coalesced reads along g, coalesced writes along i).
-__global__ void k_split_transpose(const float2* __restrict__ C, int n_in, int n, int ldA,
-                                  __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo) {
-  __shared__ float2 tile[32][33];
+// (Re C_i(g), i < Kh; Im C_i(g)), K = 2 Kh with Kh = n_in rounded up to 4,
+// through 64 (i) x 32 (g) tiles of shared memory: coalesced reads along g, 128 B
+// written per row and array.
+__global__ void __launch_bounds__(256) k_split_transpose(const float2* __restrict__ C, int n_in, int Kh, int n, int ldA,
+                                                         __nv_bfloat16* __restrict__ hi,
+                                                         __nv_bfloat16* __restrict__ lo) {
+  __shared__ float2 tile[64][33];
   const int k = blockIdx.z;
-  const int g0 = blockIdx.x * 32, i0 = blockIdx.y * 32;
-  const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
-  for (int r = ty; r < 32; r += 8) {
+  const int g0 = blockIdx.x * 32, i0 = blockIdx.y * 64;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+#pragma unroll
+  for (int r = ty; r < 64; r += 8) {
     const int i = i0 + r, g = g0 + tx;
     tile[r][tx] = (i < n_in && g < n) ? C[(static_cast<long long>(k) * n_in + i) * n + g] : make_float2(0.f, 0.f);
   }
   __syncthreads();
-  for (int r = ty; r < 32; r += 8) {
-    const int g = g0 + r, i = i0 + tx;
-    if (g >= n || i >= n_in) continue;
-    const float2 v = tile[tx][r];
-    const long long o = (static_cast<long long>(k) * n + g) * ldA;
-    __nv_bfloat16 h, l;
-    split_bf16(v.x, h, l);
-    hi[o + i] = h;
-    lo[o + i] = l;
-    split_bf16(v.y, h, l);
-    hi[o + n_in + i] = h;
-    lo[o + n_in + i] = l;
+  const int seg = 4 * (threadIdx.x & 15);
+  for (int r = threadIdx.x >> 4; r < 32; r += 16) {
+    const int g = g0 + r, i = i0 + seg;
+    if (g >= n || i >= Kh) continue;
+    float re[4], im[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 v = tile[seg + j][r];
+      re[j] = v.x;
+      im[j] = v.y;
+    }
+    const long long o = (static_cast<long long>(k) * n + g) * ldA + i;
+    uint2 h, l;
+    split4(re, h, l);
+    *reinterpret_cast<uint2*>(hi + o) = h;
+    *reinterpret_cast<uint2*>(lo + o) = l;
+    split4(im, h, l);
+    *reinterpret_cast<uint2*>(hi + o + Kh) = h;
+    *reinterpret_cast<uint2*>(lo + o + Kh) = l;
   }
 }
 
 // Rotation matrix rows for the B operand: M complex64 [k][n_in][n_out] ->
 // rows r = t*BN + part*HB + jj (output band j = t*HB + jj) of [k][rows][ld],
-// K = 2 n_in: real-output rows (Re M_ij, -Im M_ij), imaginary-output rows
+// K = 2 Kh: real-output rows (Re M_ij, -Im M_ij), imaginary-output rows
 // (Im M_ij, Re M_ij); bands >= n_out and the K padding are zero.
-__global__ void k_split_matrix(const float2* __restrict__ M, int n_in, int n_out, int HB, int rows, int ld,
+__global__ void k_split_matrix(const float2* __restrict__ M, int n_in, int Kh, int n_out, int HB, int rows, int ld,
                                __nv_bfloat16* __restrict__ hi, __nv_bfloat16* __restrict__ lo) {
   const int r = blockIdx.y, k = blockIdx.z;
   const int t = r / (2 * HB), rem = r - t * 2 * HB, part = rem / HB, j = t * HB + rem % HB;
   const long long o = (static_cast<long long>(k) * rows + r) * ld;
   for (int p = threadIdx.x; p < ld; p += blockDim.x) {
     float v = 0.f;
-    if (j < n_out && p < 2 * n_in) {
-      const int i = p < n_in ? p : p - n_in;
+    const int i = p < Kh ? p : p - Kh;
+    if (j < n_out && i < n_in) {
       const float2 m = M[(static_cast<long long>(k) * n_in + i) * n_out + j];
-      v = p < n_in ? (part ? m.y : m.x) : (part ? m.x : -m.y);
+      v = p < Kh ? (part ? m.y : m.x) : (part ? m.x : -m.y);
     }
     __nv_bfloat16 h, l;
     split_bf16(v, h, l);
@@ -508,20 +678,13 @@ int beta_split(const void* beta, int nk, int P, int n_tot, void* out, size_t out
   return QGB_OK;
 }
 
-// Pipeline depth per tile width: BN = 64 and 128 keep two CTAs per SM
-// (96 KB of stages), BN = 256 runs one CTA per SM with 4 stages (192 KB).
-template <int BN> constexpr int kStages = (BN == 64) ? 4 : (BN == 128 ? 3 : 4);
-
-// Band-block tile width for the nonlocal GEMMs.
-static int pick_bn(int nb) { return nb <= 32 ? 64 : (nb <= 64 ? 128 : 256); }
-
 struct NlWorkspace {
   long long ldB, rowsB, ldB2, partial_floats, psi_elems, b2_elems;
   int splits, kb_per_split, HB, BN;
 };
 static NlWorkspace nl_layout(int nk, int P, int nb, int n_tot) {
   NlWorkspace W;
-  W.BN = pick_bn(nb);
+  W.BN = band_tile(nb);
   W.HB = W.BN / 2;
   const long long n_tiles = (nb + W.HB - 1) / W.HB;
   W.rowsB = n_tiles * W.BN;
@@ -530,7 +693,7 @@ static NlWorkspace nl_layout(int nk, int P, int nb, int n_tot) {
   const int nkb = static_cast<int>((n_tot + BK - 1) / BK);
   const int m_tiles = static_cast<int>((2LL * P + BM - 1) / BM);
   const int tiles = m_tiles * static_cast<int>(n_tiles) * nk;
-  int splits = std::max(1, std::min(nkb, (2 * 152 + tiles - 1) / tiles));
+  const int splits = pick_splits(tiles, nkb, W.BN);
   W.kb_per_split = (nkb + splits - 1) / splits;
   W.splits = (nkb + W.kb_per_split - 1) / W.kb_per_split;
   W.partial_floats = static_cast<long long>(nk) * W.splits * m_tiles * BM * (n_tiles * W.BN);
@@ -546,7 +709,6 @@ size_t nonlocal_tc_workspace_bytes(int nk, int P, int nb, int n_tot) {
 // phases: 1 = steps 1-3 (everything that depends only on C), 2 = step 4 (the
 // accumulation into HC), 3 = both; with 4 added, step 4 stores beta (D proj)
 // into HC instead of adding it.  Phase 1 may run beside the local potential.
-template <int BN>
 static int nonlocal_tc_impl(const void* split, const void* D, int n_atoms, int pa, const void* C, void* HC,
                             void* projT, int nk, int nb, int n_tot, const NlWorkspace& W, unsigned char* ws,
                             int* err, int phases, const double* weight, cudaStream_t st) {
@@ -566,12 +728,8 @@ static int nonlocal_tc_impl(const void* split, const void* D, int n_atoms, int p
 
   if (phases & 1) {
   // 1. Wavefunctions -> bf16 hi/lo band rows.
-  {
-    dim3 grid(static_cast<unsigned>(std::min<long long>(32, (W.ldB + 255) / 256)), static_cast<unsigned>(W.rowsB), nk);
-    k_split_bands<<<grid, 256, 0, st>>>(static_cast<const float2*>(C), nb, n_tot, W.HB, static_cast<int>(W.rowsB),
-                                        static_cast<int>(W.ldB), weight, b_hi, b_lo);
-    QGB_LAUNCH_CHECK("k_split_bands");
-  }
+  int rc = launch_split_bands(C, nb, nk, n_tot, W.HB, W.rowsB, W.ldB, weight, b_hi, b_lo, st);
+  if (rc) return rc;
   // 2. <beta|psi> partials: M = 2P, N = rowsB, K = basis, split-K.
   GemmArgs g1{};
   g1.M = 2 * P;
@@ -583,7 +741,9 @@ static int nonlocal_tc_impl(const void* split, const void* D, int n_atoms, int p
   g1.part_ld = static_cast<int>(W.rowsB);
   g1.part_rows = (2LL * P + BM - 1) / BM * BM;
   g1.err = err;
-  const int rc = launch<BN, kStages<BN>, EPI_PARTIAL>(
+  g1.BN = W.BN;
+  g1.order = ORDER_SPLIT;
+  rc = launch<EPI_PARTIAL>(
       Operand{a_hi, a_lo, 2LL * P, BL.ldA, 2LL * P * BL.ldA}, Operand{b_hi, b_lo, W.rowsB, W.ldB, W.rowsB * W.ldB},
       n_tot, nk, g1, st);
   if (rc) return rc;
@@ -593,7 +753,7 @@ static int nonlocal_tc_impl(const void* split, const void* D, int n_atoms, int p
     k_reduce_proj<<<grid, dim3(32, 8), 0, st>>>(partial, W.splits, g1.part_rows, g1.part_ld, P, nb, W.HB,
                                                 weight != nullptr, static_cast<float2*>(projT));
     QGB_LAUNCH_CHECK("k_reduce_proj");
-    dim3 grid2(1, static_cast<unsigned>(W.rowsB), nk);
+    dim3 grid2(1, static_cast<unsigned>(W.rowsB / 2), nk);
     k_dapply_split<<<grid2, 256, 0, st>>>(static_cast<const float2*>(projT), static_cast<const float2*>(D),
                                           n_atoms, pa, nb, W.HB, static_cast<int>(W.rowsB),
                                           static_cast<int>(W.ldB2), b2_hi, b2_lo);
@@ -614,7 +774,9 @@ static int nonlocal_tc_impl(const void* split, const void* D, int n_atoms, int p
   g2.nb = nb;
   g2.hc_store = (phases & 4) ? 1 : 0;
   g2.err = err;
-  return launch<BN, kStages<BN>, EPI_ADD_HC>(
+  g2.BN = W.BN;
+  g2.order = ORDER_BLOCKS;
+  return launch<EPI_ADD_HC>(
       Operand{t_hi, t_lo, n_tot, BL.ldT, static_cast<long long>(n_tot) * BL.ldT},
       Operand{b2_hi, b2_lo, W.rowsB, W.ldB2, W.rowsB * W.ldB2}, 2 * P, nk, g2, st);
 }
@@ -630,17 +792,7 @@ int nonlocal_tc_phase(const void* split, const void* D, int n_atoms, int pa, con
     return fail(QGB_ERR_WORKSPACE, "nonlocal_tc workspace too small");
   const NlWorkspace W = nl_layout(nk, P, nb, n_tot);
   unsigned char* w = static_cast<unsigned char*>(ws);
-  switch (W.BN) {
-    case 64:
-      return nonlocal_tc_impl<64>(split, D, n_atoms, pa, C, HC, projT, nk, nb, n_tot, W, w, err, phases, weight,
-                                  st);
-    case 128:
-      return nonlocal_tc_impl<128>(split, D, n_atoms, pa, C, HC, projT, nk, nb, n_tot, W, w, err, phases, weight,
-                                   st);
-    default:
-      return nonlocal_tc_impl<256>(split, D, n_atoms, pa, C, HC, projT, nk, nb, n_tot, W, w, err, phases, weight,
-                                   st);
-  }
+  return nonlocal_tc_impl(split, D, n_atoms, pa, C, HC, projT, nk, nb, n_tot, W, w, err, phases, weight, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -657,17 +809,23 @@ struct GramTcLayout {
 };
 static GramTcLayout gram_tc_layout(int nk, int nx, int ny, int n) {
   GramTcLayout G;
-  const NlWorkspace W = nl_layout(nk, nx, ny, n);  // the projection's layout with P -> nx
-  G.ldA = round_up(n, 64);
+  G.BN = band_tile(ny);
+  G.HB = G.BN / 2;
+  const long long n_tiles = (ny + G.HB - 1) / G.HB, m_tiles = (2LL * nx + BM - 1) / BM;
+  G.ldA = G.ldB = round_up(n, 64);
   G.a_elems = static_cast<long long>(nk) * 2 * nx * G.ldA;
-  G.partial_floats = W.partial_floats;
-  G.psi_elems = W.psi_elems;
-  G.ldB = W.ldB;
-  G.rowsB = W.rowsB;
-  G.splits = W.splits;
-  G.kb_per_split = W.kb_per_split;
-  G.HB = W.HB;
-  G.BN = W.BN;
+  G.rowsB = n_tiles * G.BN;
+  G.psi_elems = static_cast<long long>(nk) * G.rowsB * G.ldB;
+  // The ranges of K decide how an overlap is rounded (its FP64 value holds the
+  // FP32 sums of the ranges), so they do not follow the tile width: about two
+  // per SM, over tiles of 32, 64 or 128 bands.
+  const int nkb = static_cast<int>((n + BK - 1) / BK);
+  const int bands = ny <= 32 ? 32 : (ny <= 64 ? 64 : 128);
+  const long long tiles = m_tiles * ((ny + bands - 1) / bands) * nk;
+  const int splits = static_cast<int>(std::max(1LL, std::min<long long>(nkb, (2 * 152 + tiles - 1) / tiles)));
+  G.kb_per_split = (nkb + splits - 1) / splits;
+  G.splits = (nkb + G.kb_per_split - 1) / G.kb_per_split;
+  G.partial_floats = static_cast<long long>(nk) * G.splits * m_tiles * BM * G.rowsB;
   return G;
 }
 size_t gram_tc_workspace_bytes(int nk, int nx, int ny, int n) {
@@ -677,7 +835,6 @@ size_t gram_tc_workspace_bytes(int nk, int nx, int ny, int n) {
                              round_up(2 * G.psi_elems * 2, 256)) + 1024;
 }
 
-template <int BN>
 static int gram_tc_impl(const GramTcLayout& G, const void* X, int nx, const void* Y, int ny, int nk, int n,
                         double2* out, long long out_batch, int oi, int oj, unsigned char* ws, int* err,
                         cudaStream_t st) {
@@ -689,17 +846,9 @@ static int gram_tc_impl(const GramTcLayout& G, const void* X, int nx, const void
   p += round_up(2 * G.a_elems * 2, 256);
   auto* b_hi = reinterpret_cast<__nv_bfloat16*>(p);
   auto* b_lo = b_hi + G.psi_elems;
-  {
-    dim3 grid(static_cast<unsigned>(std::min<long long>(64, (G.ldA + 255) / 256)), nx, nk);
-    k_split_beta<<<grid, 256, 0, st>>>(static_cast<const float2*>(X), nx, n, static_cast<int>(G.ldA), 0, a_hi,
-                                       a_lo, nullptr, nullptr);
-    QGB_LAUNCH_CHECK("k_split_beta");
-    dim3 grid2(static_cast<unsigned>(std::min<long long>(32, (G.ldB + 255) / 256)), static_cast<unsigned>(G.rowsB),
-               nk);
-    k_split_bands<<<grid2, 256, 0, st>>>(static_cast<const float2*>(Y), ny, n, G.HB, static_cast<int>(G.rowsB),
-                                         static_cast<int>(G.ldB), nullptr, b_hi, b_lo);
-    QGB_LAUNCH_CHECK("k_split_bands");
-  }
+  int rc = launch_split_bands(X, nx, nk, n, nx, 2LL * nx, G.ldA, nullptr, a_hi, a_lo, st);
+  if (rc) return rc;
+  if ((rc = launch_split_bands(Y, ny, nk, n, G.HB, G.rowsB, G.ldB, nullptr, b_hi, b_lo, st))) return rc;
   GemmArgs g{};
   g.M = 2 * nx;
   g.N = static_cast<int>(G.rowsB);
@@ -710,7 +859,9 @@ static int gram_tc_impl(const GramTcLayout& G, const void* X, int nx, const void
   g.part_ld = static_cast<int>(G.rowsB);
   g.part_rows = (2LL * nx + BM - 1) / BM * BM;
   g.err = err;
-  const int rc = launch<BN, kStages<BN>, EPI_PARTIAL>(
+  g.BN = G.BN;
+  g.order = ORDER_SEGMENTS;
+  rc = launch<EPI_PARTIAL>(
       Operand{a_hi, a_lo, 2LL * nx, G.ldA, 2LL * nx * G.ldA}, Operand{b_hi, b_lo, G.rowsB, G.ldB, G.rowsB * G.ldB},
       n, nk, g, st);
   if (rc) return rc;
@@ -730,11 +881,7 @@ int gram_tc(const void* X, int nx, const void* Y, int ny, int nk, int n, double2
   if (ws_bytes < gram_tc_workspace_bytes(nk, nx, ny, n)) return fail(QGB_ERR_WORKSPACE, "gram_tc workspace too small");
   const GramTcLayout G = gram_tc_layout(nk, nx, ny, n);
   unsigned char* w = static_cast<unsigned char*>(ws);
-  switch (G.BN) {
-    case 64: return gram_tc_impl<64>(G, X, nx, Y, ny, nk, n, out, out_batch, oi, oj, w, err, st);
-    case 128: return gram_tc_impl<128>(G, X, nx, Y, ny, nk, n, out, out_batch, oi, oj, w, err, st);
-    default: return gram_tc_impl<256>(G, X, nx, Y, ny, nk, n, out, out_batch, oi, oj, w, err, st);
-  }
+  return gram_tc_impl(G, X, nx, Y, ny, nk, n, out, out_batch, oi, oj, w, err, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -746,14 +893,15 @@ int gram_tc(const void* X, int nx, const void* Y, int ny, int nk, int n, double2
 // rows (B), one split-BF16x3 GEMM accumulating into out in its epilogue.
 struct RotTcLayout {
   long long ldA, a_elems, ldB, rowsB, b_elems;
-  int HB, BN;
+  int HB, BN, Kh;
 };
 static RotTcLayout rot_tc_layout(int nk, int n_in, int n_out, int n) {
   RotTcLayout R;
-  R.BN = pick_bn(n_out);
+  R.BN = band_tile(n_out);
   R.HB = R.BN / 2;
   R.rowsB = (n_out + R.HB - 1) / R.HB * static_cast<long long>(R.BN);
-  R.ldA = round_up(2LL * n_in, 64);
+  R.Kh = static_cast<int>(round_up(n_in, 4));
+  R.ldA = round_up(2LL * R.Kh, 64);
   R.ldB = R.ldA;
   R.a_elems = static_cast<long long>(nk) * n * R.ldA;
   R.b_elems = static_cast<long long>(nk) * R.rowsB * R.ldB;
@@ -765,7 +913,6 @@ size_t rotate_tc_workspace_bytes(int nk, int n_in, int n_out, int n) {
   return static_cast<size_t>(round_up(2 * R.a_elems * 2, 256) + round_up(2 * R.b_elems * 2, 256)) + 1024;
 }
 
-template <int BN>
 static int rotate_tc_impl(const RotTcLayout& R, const void* C, int n_in, int nk, int n, const void* M, int n_out,
                           void* out, bool accumulate, unsigned char* ws, int* err, cudaStream_t st) {
   unsigned char* p = reinterpret_cast<unsigned char*>(round_up(reinterpret_cast<uintptr_t>(ws), 256));
@@ -774,34 +921,34 @@ static int rotate_tc_impl(const RotTcLayout& R, const void* C, int n_in, int nk,
   p += round_up(2 * R.a_elems * 2, 256);
   auto* b_hi = reinterpret_cast<__nv_bfloat16*>(p);
   auto* b_lo = b_hi + R.b_elems;
-  // The K padding [2 n_in, ldA) of A is outside the tensor map's K extent and
-  // reads as zero; the transpose writes only the valid columns.
+  // The K padding [2 Kh, ldA) of A is outside the tensor map's K extent and
+  // reads as zero.
   {
-    dim3 grid(static_cast<unsigned>((n + 31) / 32), static_cast<unsigned>((n_in + 31) / 32), nk);
-    k_split_transpose<<<grid, dim3(32, 8), 0, st>>>(static_cast<const float2*>(C), n_in, n, static_cast<int>(R.ldA),
-                                                  a_hi, a_lo);
+    dim3 grid(static_cast<unsigned>((n + 31) / 32), static_cast<unsigned>((R.Kh + 63) / 64), nk);
+    k_split_transpose<<<grid, 256, 0, st>>>(static_cast<const float2*>(C), n_in, R.Kh, n, static_cast<int>(R.ldA), a_hi,
+                                            a_lo);
     QGB_LAUNCH_CHECK("k_split_transpose");
     dim3 grid2(1, static_cast<unsigned>(R.rowsB), nk);
-    k_split_matrix<<<grid2, 256, 0, st>>>(static_cast<const float2*>(M), n_in, n_out, R.HB,
+    k_split_matrix<<<grid2, 256, 0, st>>>(static_cast<const float2*>(M), n_in, R.Kh, n_out, R.HB,
                                           static_cast<int>(R.rowsB), static_cast<int>(R.ldB), b_hi, b_lo);
     QGB_LAUNCH_CHECK("k_split_matrix");
   }
-  if (!accumulate)
-    QGB_CUDA_CHECK(cudaMemsetAsync(out, 0, static_cast<size_t>(nk) * n_out * n * sizeof(float2), st));
   GemmArgs g{};
+  g.BN = R.BN;
+  g.order = ORDER_BLOCKS;
+  g.hc_store = accumulate ? 0 : 1;
   g.M = n;
   g.N = static_cast<int>(R.rowsB);
-  g.K = 2 * n_in;
-  g.kb_per_split = static_cast<int>((2LL * n_in + BK - 1) / BK);
+  g.K = 2 * R.Kh;
+  g.kb_per_split = static_cast<int>((2LL * R.Kh + BK - 1) / BK);
   g.splits = 1;
   g.hc = static_cast<float2*>(out);
   g.hc_batch_stride = static_cast<long long>(n_out) * n;
   g.hc_ld = n;
   g.nb = n_out;
   g.err = err;
-  return launch<BN, kStages<BN>, EPI_ADD_HC>(Operand{a_hi, a_lo, n, R.ldA, static_cast<long long>(n) * R.ldA},
-                                             Operand{b_hi, b_lo, R.rowsB, R.ldB, R.rowsB * R.ldB}, 2 * n_in, nk, g,
-                                             st);
+  return launch<EPI_ADD_HC>(Operand{a_hi, a_lo, n, R.ldA, static_cast<long long>(n) * R.ldA},
+                            Operand{b_hi, b_lo, R.rowsB, R.ldB, R.rowsB * R.ldB}, 2 * R.Kh, nk, g, st);
 }
 
 int rotate_tc(const void* C, int n_in, int nk, int n, const void* M, int n_out, void* out, bool accumulate,
@@ -819,11 +966,7 @@ int rotate_tc(const void* C, int n_in, int nk, int n, const void* M, int n_out, 
     return fail(QGB_ERR_WORKSPACE, "rotate_tc workspace too small");
   const RotTcLayout R = rot_tc_layout(nk, n_in, n_out, n);
   unsigned char* w = static_cast<unsigned char*>(ws);
-  switch (R.BN) {
-    case 64: return rotate_tc_impl<64>(R, C, n_in, nk, n, M, n_out, out, accumulate, w, err, st);
-    case 128: return rotate_tc_impl<128>(R, C, n_in, nk, n, M, n_out, out, accumulate, w, err, st);
-    default: return rotate_tc_impl<256>(R, C, n_in, nk, n, M, n_out, out, accumulate, w, err, st);
-  }
+  return rotate_tc_impl(R, C, n_in, nk, n, M, n_out, out, accumulate, w, err, st);
 }
 
 int nonlocal_tc(const void* split, const void* D, int n_atoms, int pa, const void* C, void* HC, void* projT,
@@ -852,8 +995,8 @@ int tc_wait_timeout_test(const void* ab, float* ws, int* err, unsigned long long
   g.err = err;
   g.timeout_ns = timeout_ns;
   g.skip_loads = 1;
-  return launch<64, 4, EPI_PARTIAL>(Operand{a, a, 128, 64, 128 * 64}, Operand{b, b, 64, 64, 64 * 64}, 64, 1, g,
-                                    st);
+  g.BN = 64;
+  return launch<EPI_PARTIAL>(Operand{a, a, 128, 64, 128 * 64}, Operand{b, b, 64, 64, 64 * 64}, 64, 1, g, st);
 }
 
 // Plain TN GEMM for tests: D (FP32 [M][N]) = A_hi B_hi^T + A_hi B_lo^T + A_lo B_hi^T.
@@ -873,8 +1016,9 @@ int tc_gemm_test(const void* a_hi, const void* a_lo, const void* b_hi, const voi
   g.part_ld = 64;
   g.part_rows = m_rows;
   g.err = err;
-  int rc = launch<64, 6, EPI_PARTIAL>(Operand{a_hi, a_lo, M, lda, static_cast<long long>(M) * lda},
-                                     Operand{b_hi, b_lo, N, ldb, static_cast<long long>(N) * ldb}, K, 1, g, st);
+  g.BN = 64;
+  int rc = launch<EPI_PARTIAL>(Operand{a_hi, a_lo, M, lda, static_cast<long long>(M) * lda},
+                               Operand{b_hi, b_lo, N, ldb, static_cast<long long>(N) * ldb}, K, 1, g, st);
   if (rc) return rc;
   QGB_CUDA_CHECK(cudaMemcpy2DAsync(D, N * sizeof(float), ws, 64 * sizeof(float), N * sizeof(float), M,
                                    cudaMemcpyDeviceToDevice, st));
