@@ -73,7 +73,8 @@ __global__ void __launch_bounds__(kThreads) k_xpass_batched(const qgb_batch_item
   const int r1 = static_cast<int>(local % s.N[1]);
   const long long rest = local / s.N[1];
   const int b = static_cast<int>(rest % ctx.it.nb), k = static_cast<int>(rest / ctx.it.nb);
-  body_xpass<T>(s, lp, static_cast<cplx_t<T>*>(ctx.it.planes), b, k, r1 * s.N[2], s.N[2]);
+  x_tables<T>(s, k, s.N[0] * s.N[2]);
+  body_xpass<T, false>(s, lp, static_cast<cplx_t<T>*>(ctx.it.planes), b, k, r1 * s.N[2], s.N[2]);
   QGB_BATCH_UNITS_END
 }
 

@@ -329,25 +329,41 @@ __device__ __forceinline__ void xmid_dispatch(int L1, cplx_t<T>* sm, int p, int 
   }
 }
 
+// The x-pass's items (column c < nz, sub < nsub).  W32: tiles of 32 columns, a
+// warp takes the 32 columns of a sub, so that twiddles, slab offsets and strides
+// are uniform over the warp; its lanes c >= nz (the last tile) work on columns
+// of their own that are never loaded or stored.  Otherwise columns and subs are
+// flattened over the CTA's threads.
+template <bool W32, typename F>
+__device__ __forceinline__ void x_items(int nz, int nsub, F f) {
+  if constexpr (W32) {
+    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
+    for (int sub = warp; sub < nsub; sub += blockDim.x >> 5) f(sub, static_cast<int>(threadIdx.x & 31));
+  } else {
+    const FastDiv div(nz);
+    for (int it = threadIdx.x; it < nz * nsub; it += blockDim.x) {
+      const int sub = div.quot(it);
+      f(sub, it - sub * nz);
+    }
+  }
+}
+
 // x-pass first inverse pass straight from the slab planes: item (column c,
 // sub) is the L2-point DFT over x = sub + j * L1 (natural order), read from the
 // planes at offset xs[x] (zero where no slab), times the pass-1 twiddles, stored
 // at the same shared rows.  Covers every row, so no zero fill is needed.
-template <typename T, int R>
-__device__ __forceinline__ void xpass_first_R(const cplx_t<T>* __restrict__ base, const int* xs,
-                                              int nz, int L1, int ld, int Wx, int lim) {
+template <typename T, int R, bool W32>
+__device__ __forceinline__ void xpass_first_R(const cplx_t<T>* __restrict__ base, const int* xs, int nz, int L1,
+                                              int ld, int Wx, int lim) {
   cplx_t<T>* sm = smem_c<T>();
-  const int nitems = nz * L1;
-  const FastDiv div(nz);
-  for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
-    const int sub = div.quot(it);
-    const int c = it - sub * nz;
+  x_items<W32>(nz, L1, [&](int sub, int c) {
+    const bool in = !W32 || c < nz;
     T re[R], im[R];
 #pragma unroll
     for (int j = 0; j < R; ++j) {
       const int o = xs[sub + j * L1];
       cplx_t<T> v = mk<T>(T(0), T(0));
-      if (o >= 0) v = base[static_cast<unsigned>(o + c)];
+      if (o >= 0 && in) v = base[static_cast<unsigned>(o + c)];
       re[j] = v.x;
       im[j] = v.y;
     }
@@ -360,21 +376,18 @@ __device__ __forceinline__ void xpass_first_R(const cplx_t<T>* __restrict__ base
       const int off = (sub + j * L1) * ld + c;
       if (QGB_OK_IDX(off, lim, 61)) sm[off] = value();
     });
-  }
+  });
 }
 
 // x-pass last forward pass straight to the slab planes: the L2-point DFT over
 // the shared rows sub + j * L1 gives natural x = sub + j * L1; only the rows of
 // a slab (xs[x] >= 0) are stored.
-template <typename T, int R>
-__device__ __forceinline__ void xpass_last_R(cplx_t<T>* __restrict__ base, const int* xs, int nz,
-                                             int L1, int ld, int lim) {
+template <typename T, int R, bool W32>
+__device__ __forceinline__ void xpass_last_R(cplx_t<T>* __restrict__ base, const int* xs, int nz, int L1, int ld,
+                                             int lim) {
   cplx_t<T>* sm = smem_c<T>();
-  const int nitems = nz * L1;
-  const FastDiv div(nz);
-  for (int it = threadIdx.x; it < nitems; it += blockDim.x) {
-    const int sub = div.quot(it);
-    const int c = it - sub * nz;
+  x_items<W32>(nz, L1, [&](int sub, int c) {
+    const bool in = !W32 || c < nz;
     T re[R], im[R];
 #pragma unroll
     for (int j = 0; j < R; ++j) {
@@ -389,20 +402,20 @@ __device__ __forceinline__ void xpass_last_R(cplx_t<T>* __restrict__ base, const
     x.template run<-1>();
     x.store([&](int j, auto value) {
       const int o = xs[sub + j * L1];
-      if (o >= 0) base[static_cast<unsigned>(o + c)] = value();
+      if (o >= 0 && in) base[static_cast<unsigned>(o + c)] = value();
     });
-  }
+  });
 }
 
-template <typename T, bool FIRST>
-__device__ __forceinline__ void xpass_outer(int R, cplx_t<T>* base, const int* xs, int nz, int L1,
-                                            int ld, int Wx, int lim) {
-#define QGB_XO(RR)                                                   \
-  case RR:                                                           \
-    if constexpr (FIRST)                                             \
-      xpass_first_R<T, RR>(base, xs, nz, L1, ld, Wx, lim);    \
-    else                                                             \
-      xpass_last_R<T, RR>(base, xs, nz, L1, ld, lim);         \
+template <typename T, bool FIRST, bool W32>
+__device__ __forceinline__ void xpass_outer(int R, cplx_t<T>* base, const int* xs, int nz, int L1, int ld, int Wx,
+                                            int lim) {
+#define QGB_XO(RR)                                                    \
+  case RR:                                                            \
+    if constexpr (FIRST)                                              \
+      xpass_first_R<T, RR, W32>(base, xs, nz, L1, ld, Wx, lim);       \
+    else                                                              \
+      xpass_last_R<T, RR, W32>(base, xs, nz, L1, ld, lim);            \
     break;
   switch (R) {
     QGB_XO(2) QGB_XO(3) QGB_XO(4) QGB_XO(5) QGB_XO(6) QGB_XO(7) QGB_XO(8) QGB_XO(9) QGB_XO(10) QGB_XO(12)
@@ -412,60 +425,63 @@ __device__ __forceinline__ void xpass_outer(int R, cplx_t<T>* base, const int* x
 #undef QGB_XO
 }
 
-// x-pass of the columns [c0, c0 + nz) of the N1 N2 (y, z) positions of a plane,
-// with its outer passes on the slab planes: the first inverse pass reads the slab rows from global memory
-// (L2) and the last forward pass stores the slab rows back, so shared memory
-// sees each element in three passes only (no zero fill, staging or write-back).
-// The middle step reads V(r) from global memory (it stays in L2 across the
-// bands).  An axis of a single codelet (L2 = 1) has the middle step alone and
-// is staged.  Shared layout: pencils [N0][nz] complex (threads run along the
-// columns, so rows need no padding), W_x [N0] complex, x -> slab table [N0] int:
-// 75 KB for si64 (96^3) in FP32, so 3 CTAs fit an SM.
+// The x-pass's tables behind `lim` elements of data: W_x [N0] complex, x -> plane
+// offset [N0] int (-1: no slab).  Ends with __syncthreads().
 template <typename T>
+__device__ __forceinline__ void x_tables(const qgb_sphere& s, const int k, const int lim) {
+  const int N0 = s.N[0];
+  int* xs = reinterpret_cast<int*>(smem_c<T>() + lim + N0);
+  load_twiddles<T>(lim, static_cast<const cplx_t<T>*>(s.twiddle) + s.tw_off[0], N0);
+  for (int x = threadIdx.x; x < N0; x += blockDim.x) xs[x] = -1;
+  __syncthreads();
+  const int* i0 = s.slab_i0 + k * s.max_slabs;
+  for (int sl = threadIdx.x; sl < s.n_slabs[k]; sl += blockDim.x) {
+    const int x = i0[sl];
+    if (QGB_OK_IDX(x, N0, 63)) xs[x] = sl * s.N[1] * s.N[2];
+  }
+  __syncthreads();
+}
+
+// x-pass of the columns [c0, c0 + nz) of the N1 N2 (y, z) positions of a plane,
+// with its outer passes on the slab planes: the first inverse pass reads the
+// slab rows from global memory (L2) and the last forward pass stores the slab
+// rows back, so shared memory sees each element in three passes only (no zero
+// fill, staging or write-back).  The middle step reads V(r) from global memory
+// (it stays in L2 across the bands).  An axis of a single codelet (L2 = 1) has
+// the middle step alone and is staged.  Shared layout: pencils [N0][ld] complex
+// (ld = 32 for W32, else nz; threads run along the columns, so rows need no
+// padding), then x_tables.
+template <typename T, bool W32>
 __device__ __forceinline__ void body_xpass(const qgb_sphere& s, const LocalParams& lp, cplx_t<T>* __restrict__ planes,
                                            const int b, const int k, const int c0, const int nz) {
   using C2 = cplx_t<T>;
-  const int N0 = s.N[0], N1 = s.N[1], N2 = s.N[2], ld = nz;
+  const int N0 = s.N[0], N1 = s.N[1], N2 = s.N[2], ld = W32 ? 32 : nz;
   const int L1 = s.L1[0], L2 = s.L2[0];
   const int lim = N0 * ld, Wx = lim;
   C2* sm = smem_c<T>();
   int* xs = reinterpret_cast<int*>(sm + Wx + N0);
-  const C2* tw = static_cast<const C2*>(s.twiddle);
-  load_twiddles<T>(Wx, tw + s.tw_off[0], N0);
-  for (int x = threadIdx.x; x < N0; x += blockDim.x) xs[x] = -1;
-  __syncthreads();
-  const int nslabs = s.n_slabs[k];
-  const int* i0 = s.slab_i0 + k * s.max_slabs;
-  for (int sl = threadIdx.x; sl < nslabs; sl += blockDim.x) {
-    const int x = i0[sl];
-    if (QGB_OK_IDX(x, N0, 63)) xs[x] = sl * N1 * N2;
-  }
-  __syncthreads();
   const size_t plane = static_cast<size_t>(N1) * N2;
   C2* base = planes + plane_index(s, k, b, lp.nb, 0) * plane + c0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   if (L2 > 1) {
-    xpass_outer<T, true>(L2, base, xs, nz, L1, ld, Wx, lim);
+    xpass_outer<T, true, W32>(L2, base, xs, nz, L1, ld, Wx, lim);
   } else {
     for (int x = warp; x < N0; x += nwarps) {
       const int o = xs[x];
-      for (int c = lane; c < nz; c += 32) sm[x * ld + c] = o >= 0 ? base[o + c] : mk<T>(T(0), T(0));
+      for (int c = lane; c < ld; c += 32) sm[x * ld + c] = o >= 0 && c < nz ? base[o + c] : mk<T>(T(0), T(0));
     }
   }
   __syncthreads();
   // V[p0][c0 + c] with p0 = a * L1 + j: j-stride N1 * N2.
   const T* V = static_cast<const T*>(s.V) + c0;
-  const FastDiv div(nz);
-  for (int it = threadIdx.x; it < nz * L2; it += blockDim.x) {
-    const int a = div.quot(it);
-    const int c = it - a * nz;
-    if (!QGB_OK_IDX(c + (a * L1 + L1 - 1) * ld, lim, 7) || !QGB_OK_IDX((L1 - 1) * L2 + a, N0, 9)) continue;
-    xmid_dispatch<T>(L1, sm, c + a * L1 * ld, ld, V + static_cast<unsigned>(a * L1 * N1 * N2 + c),
+  x_items<W32>(nz, L2, [&](int a, int c) {
+    if (!QGB_OK_IDX(c + (a * L1 + L1 - 1) * ld, lim, 7) || !QGB_OK_IDX((L1 - 1) * L2 + a, N0, 9)) return;
+    xmid_dispatch<T>(L1, sm, c + a * L1 * ld, ld, V + static_cast<unsigned>(a * L1 * N1 * N2 + (W32 ? min(c, nz - 1) : c)),
                      N1 * N2, Wx, L2, a);
-  }
+  });
   __syncthreads();
   if (L2 > 1) {
-    xpass_outer<T, false>(L2, base, xs, nz, L1, ld, Wx, lim);
+    xpass_outer<T, false, W32>(L2, base, xs, nz, L1, ld, Wx, lim);
   } else {
     for (int x = warp; x < N0; x += nwarps) {
       const int o = xs[x];
@@ -584,12 +600,18 @@ __global__ void __launch_bounds__(kMaxThreadsYZ<T>, sizeof(T) == 4 ? 2 : 1) k_if
   body_ifft_yz<T>(s, lp, C, planes, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
-// A tile of `nc` columns per CTA.
+// `tiles` tiles of 32 columns per CTA, one after the other.
 template <typename T>
 __global__ void __launch_bounds__(kThreads, kCtasX<T>) k_xpass(const qgb_sphere s, LocalParams lp,
-                                                            cplx_t<T>* __restrict__ planes, int nc) {
-  const int c0 = blockIdx.x * nc;
-  body_xpass<T>(s, lp, planes, blockIdx.y, blockIdx.z, c0, min(nc, s.N[1] * s.N[2] - c0));
+                                                            cplx_t<T>* __restrict__ planes, int tiles) {
+  x_tables<T>(s, blockIdx.z, 32 * s.N[0]);
+  const int cols = s.N[1] * s.N[2];
+  if (sizeof(T) == 8) tiles = 1;  // (the loop costs FP64 4%)
+  int c0 = blockIdx.x * tiles * 32;
+  for (int t = 0; t < tiles && c0 < cols; ++t, c0 += 32) {
+    if (t > 0) __syncthreads();  // the tile's shared memory is reused
+    body_xpass<T, true>(s, lp, planes, blockIdx.y, blockIdx.z, c0, min(32, cols - c0));
+  }
 }
 
 // C and out may alias (in-place apply): no __restrict__ on them.
@@ -648,34 +670,32 @@ template <typename T> int threads_yz(const qgb_sphere& s, int nb) {
   return threads;
 }
 
-// Tile of columns and CTA size of the x-pass.  A plane's N1 N2 columns are one
-// contiguous range, so a tile need not be a y-row: it is the one for which the
-// passes fill their rounds of the CTA's threads (nc L1 items of radix L2 twice,
-// nc L2 items of radix L1 in both directions), by launch_cost; a CTA's tables
-// and barriers count 8 and its share of them.  Tiles below 32 columns (256 B of
-// a row) load worse.
-// Measured against whole y-rows (us, FP32): si64 (96^3, 160 bands; a row of 96 in
-// 5 + 3 rounds of 256 threads, a tile of 32 in 3 + 2 full ones of 128) 436 ->
-// 416; 36^3, 144 bands (216 items a row) 38 -> 25; 72^3, 800 bands 1046 -> 856.
-template <typename T> void x_tile(const qgb_sphere& s, int nb, int* nc, int* threads) {
-  const int cols = s.N[1] * s.N[2], L1 = s.L1[0], L2 = s.L2[0];
+// CTA size of the x-pass and the tiles a CTA takes.  A plane's N1 N2 columns are
+// one contiguous range, so its tiles need not be y-rows: they are 32 columns
+// (256 B of a row in FP32), and the warps take the L1 subs of the outer passes
+// (radix L2, twice) and the L2 of the middle step (radix L1, both directions) in
+// as few rounds as launch_cost allows.  si64 (96^3): 3 + 2 full rounds of 4 warps.
+// In FP32 up to 8 tiles share a CTA's tables while 4 waves of CTAs are left.
+// Measured against whole y-rows flattened over 256 threads (x-pass, us): si64, 160
+// bands 436 -> 377 (FP64, 32 bands 592 -> 568), 36^3, 144 bands 38 -> 21 (FP64 177 ->
+// 136), 72^3, 800 bands 1046 -> 862.
+template <typename T> void x_shape(const qgb_sphere& s, int nb, int* threads, int* tiles) {
+  const int L1 = s.L1[0], L2 = s.L2[0];
+  const size_t smem = x_smem_bytes(s, 32, sizeof(cplx_t<T>));
+  const double total = (static_cast<double>(s.N[1]) * s.N[2] + 31) / 32 * nb * s.nk;
   double best = 1e30;
-  *nc = std::min(cols, 32);
   *threads = 128;
-  for (int c = 32; c <= 256; c += 16) {
-    const size_t smem = x_smem_bytes(s, c, sizeof(cplx_t<T>));
-    if (c > 32 && (smem > kSmemPerSm || c >= cols + 16)) break;
-    for (int t = 64; t <= kThreads; t += 32) {
-      const int outer = L2 > 1 ? (c * L1 + t - 1) / t : 0, mid = (c * L2 + t - 1) / t;
-      const double work = 2.0 * (outer * L2 + mid * L1) + 8.0 + 4.0 * s.N[0] / t;
-      const double cost = launch_cost<T>(static_cast<double>((cols + c - 1) / c) * nb * s.nk, t, smem, work);
-      if (cost < best * 0.999) {
-        best = cost;
-        *nc = std::min(c, cols);
-        *threads = t;
-      }
+  for (int w = 1; w <= kThreads / 32; ++w) {
+    const int outer = L2 > 1 ? (L1 + w - 1) / w : 0, mid = (L2 + w - 1) / w;
+    const double work = 2.0 * (outer * L2 + mid * L1) + 8.0;
+    const double cost = launch_cost<T>(total, 32 * w, smem, work);
+    if (cost < best * 0.999) {
+      best = cost;
+      *threads = 32 * w;
     }
   }
+  const int ctas = std::max(1, (sizeof(T) == 4 ? 768 : 512) / *threads);
+  *tiles = sizeof(T) == 8 ? 1 : std::max(1, std::min(8, static_cast<int>(total / (4.0 * 152.0 * ctas))));
 }
 
 template <typename T>
@@ -694,11 +714,12 @@ int launch_chunk(const qgb_sphere& s, const LocalParams& lp, const void* C, void
   using C2 = cplx_t<T>;
   int rc;
   if ((rc = launch_ifft_yz<T>(s, lp, C, planes, st))) return rc;
-  int nc, tx;
-  x_tile<T>(s, lp.nb, &nc, &tx);
-  const size_t smx = x_smem_bytes(s, nc, sizeof(C2));
+  const size_t smx = x_smem_bytes(s, 32, sizeof(C2));
   if ((rc = raise_smem_limit(k_xpass<T>, smx))) return rc;
-  k_xpass<T><<<dim3((s.N[1] * s.N[2] + nc - 1) / nc, lp.nb, s.nk), tx, smx, st>>>(s, lp, static_cast<C2*>(planes), nc);
+  int tx, tiles;
+  x_shape<T>(s, lp.nb, &tx, &tiles);
+  k_xpass<T><<<dim3((s.N[1] * s.N[2] + 32 * tiles - 1) / (32 * tiles), lp.nb, s.nk), tx, smx, st>>>(
+      s, lp, static_cast<C2*>(planes), tiles);
   QGB_LAUNCH_CHECK("k_xpass");
   if (gather_after) QGB_CUDA_CHECK(cudaStreamWaitEvent(st, gather_after, 0));
   const size_t smem = yz_smem_bytes(s, sizeof(C2));
