@@ -22,13 +22,20 @@ CODELET_SIZES = (1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 14, 15, 16)
 
 
 def factor_axis(N: int, prefer: tuple | None = None) -> tuple[int, int]:
-    """(L1, L2) with L1 * L2 = N, both codelet sizes: one pass when N is itself a
-    codelet size, else the most balanced split with L1 >= L2."""
+    """(L1, L2) with L1 * L2 = N, both codelet sizes: the most balanced split with
+    L1 >= L2, one pass for N < 8 and for N with no such split.
+
+    A codelet of 8 or more gives a plane few, long items: axes of 8 to 16 leave
+    most of a CTA idle with one pass and fill it with two.  Local potential on
+    N^3 grids, 12 bands, one pass -> two, us: FP64 8: 24 -> 20, 9: 29 -> 20,
+    10: 31 -> 23, 12: 34 -> 22, 14: 45 -> 29, 16: 40 -> 22; FP32 8: 13.9 -> 13.0,
+    10: 15.3 -> 13.9, 12: 17.5 -> 13.4, 16: 19.3 -> 13.4.  128 bands of 16^3:
+    FP64 61 -> 42, FP32 22 -> 16."""
     if prefer is not None:
         if prefer[0] * prefer[1] != N or prefer[0] not in CODELET_SIZES or prefer[1] not in CODELET_SIZES:
             raise ValueError(f"bad factorisation {prefer} for N={N}")
         return tuple(prefer)
-    if N in CODELET_SIZES:
+    if N < 8 and N in CODELET_SIZES:
         return (N, 1)
     best = None
     for L1 in CODELET_SIZES:
