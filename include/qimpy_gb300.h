@@ -282,7 +282,8 @@ int qgb_matmul_ws(int dtype, const void* C, int n_in, int nk, int n_tot, const v
  * out[k][b][g] += sum_p beta[k][p][g] (D_all projT[k][b])[p]  (replaces
  * beta @ (D_all @ C.proj), qimpy/dft/electrons/_hamiltonian.py:22-24 with
  * Wavefunction.matmul, _wavefunction_dot.py:137-191).  D is given per atom
- * block (n_atoms blocks of pa x pa).  `work` holds nk*nb*P complex values.
+ * block (n_atoms blocks of pa x pa).  `work` holds nk*nb*P complex values (scratch: small
+ * products leave it untouched).
  */
 int qgb_apply_nonlocal(int dtype, const void* beta, const void* D, int n_atoms, int pa,
                        const void* projT, void* out, int nk, int nb, int n_tot, void* work,

@@ -180,7 +180,7 @@ __global__ void k_gram_reduce(const cplx_t<T>* __restrict__ partial, int splits,
 // sums are folded across the lanes (each step halves the values a lane keeps,
 // so TI TJ complex sums cost about as many additions) and then the 8 warps.
 // The 64 x 64 tiles above would multiply padding and leave most SMs idle (k = 8
-// times 8 x 18 outputs over 1150 g: 517 us against 16 us here).
+// times 8 x 18 outputs over 1150 g: 517 us against 14 us here).
 template <typename T, typename OutT, int TI, int TJ>
 __global__ void __launch_bounds__(256) k_gram_small(const GramArgs a) {
   using C2 = cplx_t<T>;
@@ -375,19 +375,40 @@ __global__ void __launch_bounds__(256) k_rotate(const RotArgs a) {
   }
 }
 
-// Small rotations: one g and 4 j a thread, W broadcast.  (The 32 x 128 tiles
+// Small rotations: one g and TJ j a thread, W broadcast.  (The 32 x 128 tiles
 // above multiply padding and fill few SMs: 71 us for 8 x 18 over 1150 g and 8 k.)
-template <typename T>
-__global__ void __launch_bounds__(64) k_rotate_small(const RotArgs a) {
+// The FP64 pipe's 2 multiply-adds a clock and SM bound it, so the SM with the
+// most threads times outputs does: the host picks TJ and the CTA size by that
+// (pick_rotate_small; 10.9 -> 5.1 us for 12 x 6 over 300 g and 2 k, where CTAs of
+// 64 x 4 would occupy 20 SMs).
+// NL, the back-projection: W(i, j) = sum_c D[atom(i)][i % pa][c] proj[j][c], put in
+// shared memory by each CTA for its TJ columns.  It repeats pa of every 64 (32)
+// multiply-adds and saves k_dapply and its launch (3 to 4 us).
+template <typename T, int TJ, bool NL>
+__global__ void __launch_bounds__(64) k_rotate_small(const RotArgs a, const cplx_t<T>* __restrict__ D, int pa) {
   using C2 = cplx_t<T>;
-  constexpr int TJ = 4;
-  const int g = blockIdx.x * 64 + threadIdx.x, j0 = blockIdx.y * TJ, k = blockIdx.z;
+  extern __shared__ __align__(16) unsigned char small_smem[];
+  C2* Ws = reinterpret_cast<C2*>(small_smem);  // [TJ][Kin]
+  const int g = blockIdx.x * blockDim.x + threadIdx.x, j0 = blockIdx.y * TJ, k = blockIdx.z;
+  const C2* Wk = static_cast<const C2*>(a.W) + k * a.w_batch;
+  if constexpr (NL) {
+    for (int e = threadIdx.x; e < TJ * a.Kin; e += blockDim.x) {
+      const int p = e / a.Kin, i = e - p * a.Kin, atom = i / pa;
+      const C2* x = Wk + static_cast<long long>(min(j0 + p, a.Nout - 1)) * a.wj + atom * pa;
+      const C2* d = D + static_cast<long long>(i) * pa;
+      C2 acc = mk<T>(T(0), T(0));
+      for (int c = 0; c < pa; ++c) cmac<T>(acc, d[c], x[c]);
+      Ws[e] = acc;
+    }
+    __syncthreads();
+  }
   if (g >= a.G) return;
   const C2* X = static_cast<const C2*>(a.X) + k * a.x_batch + g;
   const C2* W[TJ];
 #pragma unroll
   for (int p = 0; p < TJ; ++p)
-    W[p] = static_cast<const C2*>(a.W) + k * a.w_batch + static_cast<long long>(min(j0 + p, a.Nout - 1)) * a.wj;
+    W[p] = NL ? Ws + p * a.Kin : Wk + static_cast<long long>(min(j0 + p, a.Nout - 1)) * a.wj;
+  const long long wi = NL ? 1 : a.wi;
   C2 acc[TJ];
 #pragma unroll
   for (int p = 0; p < TJ; ++p) acc[p] = mk<T>(T(0), T(0));
@@ -395,7 +416,7 @@ __global__ void __launch_bounds__(64) k_rotate_small(const RotArgs a) {
   for (int i = 0; i < a.Kin; ++i) {
     const C2 x = X[static_cast<long long>(i) * a.ldx];
 #pragma unroll
-    for (int p = 0; p < TJ; ++p) cmac<T>(acc[p], W[p][static_cast<long long>(i) * a.wi], x);
+    for (int p = 0; p < TJ; ++p) cmac<T>(acc[p], W[p][i * wi], x);
   }
   C2* out = static_cast<C2*>(a.out) + k * a.out_batch + g;
 #pragma unroll
@@ -461,18 +482,62 @@ static bool small_product(int nk, int M, int N, int K) {
   return static_cast<double>(nk) * M * N * K < 3e6 && nk <= 65535;
 }
 
-// The largest of the 4 x 4, 2 x 4 and 2 x 2 outputs a CTA that gives every SM one.
+// Work of the SM that gets the most of `ctas` equal CTAs.  `work` counts an
+// output's multiply-add as 1 in FP64 (2 a clock and SM, nothing else is near);
+// in FP32 the loads cost more than the multiply-adds, so larger tiles are kept
+// longer.
+static long long most_loaded(long long ctas, int work) { return (ctas + kSms - 1) / kSms * work; }
+
+// The tile that loads the fullest SM least, the larger one on a tie: 8 x 18
+// outputs of 8 k are 160 tiles of 2 x 4, two on 8 of the SMs, or 288 of 2 x 2,
+// also two but half the size (1150 g, FP64: 23.7 -> 13.6 us).
 template <typename T, typename OutT>
 static void launch_gram_small(const GramArgs& g, int nk, cudaStream_t st) {
   const auto ctas = [&](int ti, int tj) {
     return static_cast<unsigned>((g.M + ti - 1) / ti) * static_cast<unsigned>((g.N + tj - 1) / tj);
   };
-  if (static_cast<long long>(ctas(4, 4)) * nk >= kSms)
+  const auto cost = [&](int ti, int tj) {
+    return most_loaded(static_cast<long long>(ctas(ti, tj)) * nk,
+                       sizeof(T) == 8 ? ti * tj : ti * tj + 2 * (ti + tj));
+  };
+  if (cost(4, 4) <= std::min(cost(2, 4), cost(2, 2)))
     k_gram_small<T, OutT, 4, 4><<<dim3(ctas(4, 4), nk), 256, 0, st>>>(g);
-  else if (static_cast<long long>(ctas(2, 4)) * nk >= kSms)
+  else if (cost(2, 4) <= cost(2, 2))
     k_gram_small<T, OutT, 2, 4><<<dim3(ctas(2, 4), nk), 256, 0, st>>>(g);
   else
     k_gram_small<T, OutT, 2, 2><<<dim3(ctas(2, 2), nk), 256, 0, st>>>(g);
+}
+
+// Columns a thread and threads a CTA of k_rotate_small, by the same rule: 4, 2 or
+// 1 columns of 64 threads, or 1 of 32.
+struct RotSmall {
+  int tj, threads;
+};
+static RotSmall pick_rotate_small(int dtype, int nk, int Nout, int G) {
+  RotSmall best{4, 64};
+  long long least = -1;
+  for (const RotSmall c : {RotSmall{4, 64}, RotSmall{2, 64}, RotSmall{1, 64}, RotSmall{1, 32}}) {
+    const long long ctas = static_cast<long long>((G + c.threads - 1) / c.threads) * ((Nout + c.tj - 1) / c.tj) * nk;
+    const long long cost = most_loaded(ctas, c.threads * (dtype == QGB_F64 ? c.tj : 2 * c.tj + 2));
+    if ((Nout + c.tj - 1) / c.tj <= 65535 && (least < 0 || cost < least)) {
+      least = cost;
+      best = c;
+    }
+  }
+  return best;
+}
+
+template <typename T, bool NL>
+static void launch_rotate_small(const RotArgs& r, int nk, const void* D, int pa, RotSmall c, cudaStream_t st) {
+  const dim3 grid((r.G + c.threads - 1) / c.threads, (r.Nout + c.tj - 1) / c.tj, nk);
+  const size_t smem = NL ? static_cast<size_t>(c.tj) * r.Kin * sizeof(cplx_t<T>) : 0;
+  const cplx_t<T>* d = static_cast<const cplx_t<T>*>(D);
+  if (c.tj == 4)
+    k_rotate_small<T, 4, NL><<<grid, c.threads, smem, st>>>(r, d, pa);
+  else if (c.tj == 2)
+    k_rotate_small<T, 2, NL><<<grid, c.threads, smem, st>>>(r, d, pa);
+  else
+    k_rotate_small<T, 1, NL><<<grid, c.threads, smem, st>>>(r, d, pa);
 }
 
 // out(i, j) of type out_dtype (complex) = sum_g conj(A(i, g)) B(j, g), per k.
@@ -545,11 +610,11 @@ int rotate(int dtype, const void* X, long long x_batch, int ldx, const void* W, 
     return oz_rotate(X, x_batch, ldx, W, w_batch, wi, wj, nk, Kin, Nout, G, out, out_batch, ldo, accumulate, ws, st);
   RotArgs r{X, W, out, x_batch, w_batch, out_batch, ldx, ldo, wi, wj, Kin, Nout, G, accumulate ? 1 : 0};
   if (small_product(nk, Kin, Nout, G) && (Nout + 3) / 4 <= 65535 && (dtype == QGB_F64 || dtype == QGB_F32)) {
-    const dim3 grid((G + 63) / 64, (Nout + 3) / 4, nk);
+    const RotSmall c = pick_rotate_small(dtype, nk, Nout, G);
     if (dtype == QGB_F64)
-      k_rotate_small<double><<<grid, 64, 0, st>>>(r);
+      launch_rotate_small<double, false>(r, nk, nullptr, 0, c, st);
     else
-      k_rotate_small<float><<<grid, 64, 0, st>>>(r);
+      launch_rotate_small<float, false>(r, nk, nullptr, 0, c, st);
     QGB_LAUNCH_CHECK("k_rotate_small");
     return QGB_OK;
   }
@@ -565,6 +630,25 @@ int rotate(int dtype, const void* X, long long x_batch, int ldx, const void* W, 
     return fail(QGB_ERR_INVALID, "unknown dtype %d", dtype);
   }
   QGB_LAUNCH_CHECK("k_rotate");
+  return QGB_OK;
+}
+
+bool backproject_small_use(int nk, int n_atoms, int pa, int nb, int n_tot) {
+  const long long P = static_cast<long long>(n_atoms) * pa;
+  return pa <= 8 && P <= 512 && small_product(nk, static_cast<int>(P), nb, n_tot) && (nb + 3) / 4 <= 65535;
+}
+
+int backproject_small(int dtype, const void* beta, const void* D, int n_atoms, int pa, const void* projT, void* out,
+                      int nk, int nb, int n_tot, cudaStream_t st) {
+  const int P = n_atoms * pa;
+  const RotArgs r{beta, projT, out, static_cast<long long>(P) * n_tot, static_cast<long long>(nb) * P,
+                  static_cast<long long>(nb) * n_tot, n_tot, n_tot, 1, P, P, nb, n_tot, 1};
+  const RotSmall c = pick_rotate_small(dtype, nk, nb, n_tot);
+  if (dtype == QGB_F64)
+    launch_rotate_small<double, true>(r, nk, D, pa, c, st);
+  else
+    launch_rotate_small<float, true>(r, nk, D, pa, c, st);
+  QGB_LAUNCH_CHECK("k_rotate_small");
   return QGB_OK;
 }
 

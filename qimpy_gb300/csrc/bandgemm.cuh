@@ -42,4 +42,12 @@ int oz_rotate(const void* X, long long x_batch, int ldx, const void* W, long lon
 int dapply(int dtype, const void* proj, const void* D, int n_atoms, int pa, int nb, int nk, void* Dp,
            cudaStream_t st);
 
+// out[k][b][g] += sum_p beta[k][p][g] (D projT[k][b])[p] in one launch, D applied
+// by every CTA: for products of `rotate`'s small kernel with blocks of at most 8
+// (an eighth more multiply-adds, about what the launch saved costs at 3e6) and at
+// most 512 projectors (32 KB of shared memory).
+bool backproject_small_use(int nk, int n_atoms, int pa, int nb, int n_tot);
+int backproject_small(int dtype, const void* beta, const void* D, int n_atoms, int pa, const void* projT, void* out,
+                      int nk, int nb, int n_tot, cudaStream_t st);
+
 }  // namespace qgb

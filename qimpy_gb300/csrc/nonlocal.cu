@@ -33,7 +33,9 @@ int apply_nonlocal(int dtype, const void* beta, const void* D, int n_atoms, int 
     return fail(QGB_ERR_INVALID, "bad apply_nonlocal sizes");
   if (nk == 0 || P == 0 || nb == 0) return QGB_OK;
   if (!beta || !D || !projT || !out || !work) return fail(QGB_ERR_INVALID, "NULL pointer in apply_nonlocal");
-  int rc = dapply(dtype, projT, D, n_atoms, pa, nb, nk, work, st);
+  if (backproject_small_use(nk, n_atoms, pa, nb, n_tot))
+    return backproject_small(dtype, beta, D, n_atoms, pa, projT, out, nk, nb, n_tot, st);
+  const int rc = dapply(dtype, projT, D, n_atoms, pa, nb, nk, work, st);
   if (rc) return rc;
   // out[k][b][g] += sum_p beta[k][p][g] Dp[k][b][p]: i = p, j = b, W(p, b) = Dp[b*P + p].
   return rotate(dtype, beta, static_cast<long long>(P) * n_tot, n_tot, work, static_cast<long long>(nb) * P, 1, P,
