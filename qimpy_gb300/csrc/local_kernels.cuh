@@ -8,6 +8,7 @@
 #include <cmath>
 
 #include "fft_steps.cuh"
+#include "packed_f32.cuh"
 
 namespace qgb {
 
@@ -491,6 +492,203 @@ __device__ __forceinline__ void body_xpass(const qgb_sphere& s, const LocalParam
   }
 }
 
+// ---------------------------------------------------------------------------
+// The FP32 x-pass on tiles of 64 columns: a lane takes columns c and c + 32 as a
+// packed pair (packed_f32.cuh).  Otherwise as body_xpass<T, true>: the same
+// passes, rows and items, with shared elements of 16 B and the twiddles doubled.
+// One column a lane was bound by instruction issue (2.5 of 4 a clock): pairs
+// issue 25.0 M instead of 35.8 M for 40 bands of 72^3.  What they need in return
+// is that a thread's loads are all in flight before the first is used (loads and
+// packing in one loop: 465 us instead of 360 at si64) and five CTAs' worth of
+// warps at 96 registers (x_max_threads).  x-pass, us: 72^3, 800 bands 862 -> 751,
+// 96^3, 160 bands 377 -> 367, 36^3, 144 bands 21.7 -> 20.3.
+// ---------------------------------------------------------------------------
+
+__device__ __forceinline__ cpair_t* smem_pairs() { return reinterpret_cast<cpair_t*>(qgb_smem); }
+
+// The columns of a lane that the tile has (the last tile of a plane is ragged).
+struct PairLane {
+  int c;
+  bool in0, in1;
+};
+
+__device__ __forceinline__ cpair_t pair_load(const float2* __restrict__ row, const PairLane l) {
+  float2 a = make_float2(0.0f, 0.0f), b = a;
+  if (l.in0) a = row[l.c];
+  if (l.in1) b = row[l.c + 32];
+  return make_ulonglong2(pair_of(a.x, b.x), pair_of(a.y, b.y));
+}
+__device__ __forceinline__ void pair_store(float2* __restrict__ row, const PairLane l, pair_t re, pair_t im) {
+  const float2 x = pair_split(re), y = pair_split(im);
+  if (l.in0) row[l.c] = make_float2(x.x, y.x);
+  if (l.in1) row[l.c + 32] = make_float2(x.y, y.y);
+}
+
+template <int R>
+__device__ __forceinline__ void xpair_first_R(const float2* __restrict__ base, const int* xs, const PairLane l, int L1,
+                                              int Wx, int lim) {
+  cpair_t* sm = smem_pairs();
+  x_items<true>(0, L1, [&](int sub, int c) {
+    PairBlock<R> x;
+    float2 p[R], q[R];  // all loads in flight before the first is used
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const int o = xs[sub + j * L1];
+      p[j] = q[j] = make_float2(0.0f, 0.0f);
+      if (o >= 0 && l.in0) p[j] = base[static_cast<unsigned>(o + c)];
+      if (o >= 0 && l.in1) q[j] = base[static_cast<unsigned>(o + c + 32)];
+    }
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      x.re[j] = F2::of(pair_of(p[j].x, q[j].x));
+      x.im[j] = F2::of(pair_of(p[j].y, q[j].y));
+    }
+    x.template run<+1>();
+#pragma unroll
+    for (int j = 1; j < R; ++j) x.template twiddle<+1>(j, sm[Wx + sub * R + j]);
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const int off = (sub + j * L1) * 32 + c;
+      if (QGB_OK_IDX(off, lim, 61)) sm[off] = make_ulonglong2(x.re[j].value(), x.im[j].value());
+    }
+  });
+}
+
+template <int R>
+__device__ __forceinline__ void xpair_last_R(float2* __restrict__ base, const int* xs, const PairLane l, int L1,
+                                             int lim) {
+  const cpair_t* sm = smem_pairs();
+  x_items<true>(0, L1, [&](int sub, int c) {
+    PairBlock<R> x;
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const int off = (sub + j * L1) * 32 + c;
+      if (!QGB_OK_IDX(off, lim, 62)) return;
+      const cpair_t v = sm[off];
+      x.re[j] = F2::of(v.x);
+      x.im[j] = F2::of(v.y);
+    }
+    x.template run<-1>();
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const int o = xs[sub + j * L1];
+      if (o >= 0) pair_store(base + static_cast<unsigned>(o), l, x.re[j].value(), x.im[j].value());
+    }
+  });
+}
+
+template <int R>
+__device__ __forceinline__ void xpair_mid_R(const float* __restrict__ V, const PairLane l, unsigned plane, int L2,
+                                            int Wx, int lim) {
+  cpair_t* sm = smem_pairs();
+  const int v0 = l.in0 ? l.c : 0, v1 = l.in1 ? l.c + 32 : v0;  // lanes beyond the tile read V of its first columns
+  x_items<true>(0, L2, [&](int a, int c) {
+    if (!QGB_OK_IDX(c + (a * R + R - 1) * 32, lim, 7)) return;
+    cpair_t* p = sm + a * R * 32 + c;
+    const float* Va = V + static_cast<unsigned>(a * R) * plane;
+    PairBlock<R> x;
+    pair_t v[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      const cpair_t e = p[j * 32];
+      x.re[j] = F2::of(e.x);
+      x.im[j] = F2::of(e.y);
+    }
+    float f0[R], f1[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      f0[j] = Va[j * plane + v0];
+      f1[j] = Va[j * plane + v1];
+    }
+#pragma unroll
+    for (int j = 0; j < R; ++j) v[j] = pair_of(f0[j], f1[j]);
+    x.template run<+1>();
+#pragma unroll
+    for (int j = 0; j < R; ++j) x.scale(j, v[j]);
+    x.template run<-1>();
+    if (L2 > 1) {
+#pragma unroll
+      for (int j = 1; j < R; ++j) x.template twiddle<-1>(j, sm[Wx + j * L2 + a]);
+    }
+#pragma unroll
+    for (int j = 0; j < R; ++j) p[j * 32] = make_ulonglong2(x.re[j].value(), x.im[j].value());
+  });
+}
+
+// STEP 0: first inverse pass (radix L2), 1: middle step (L1), 2: last forward (L2).
+template <int STEP>
+__device__ __forceinline__ void xpair_step(int R, float2* base, const float* V, const int* xs, const PairLane l,
+                                           unsigned plane, int L1, int L2, int Wx, int lim) {
+#define QGB_XP(RR)                                             \
+  case RR:                                                     \
+    if constexpr (STEP == 0)                                   \
+      xpair_first_R<RR>(base, xs, l, L1, Wx, lim);             \
+    else if constexpr (STEP == 1)                              \
+      xpair_mid_R<RR>(V, l, plane, L2, Wx, lim);               \
+    else                                                       \
+      xpair_last_R<RR>(base, xs, l, L1, lim);                  \
+    break;
+  switch (R) {
+    QGB_XP(1) QGB_XP(2) QGB_XP(3) QGB_XP(4) QGB_XP(5) QGB_XP(6) QGB_XP(7) QGB_XP(8) QGB_XP(9) QGB_XP(10) QGB_XP(12)
+    QGB_XP(14) QGB_XP(15) QGB_XP(16)
+    default: break;
+  }
+#undef QGB_XP
+}
+
+// As x_tables, behind 32 N0 pairs.
+__device__ __forceinline__ void x_tables_pair(const qgb_sphere& s, const int k) {
+  const int N0 = s.N[0];
+  cpair_t* W = smem_pairs() + 32 * N0;
+  int* xs = reinterpret_cast<int*>(W + N0);
+  const float2* tw = static_cast<const float2*>(s.twiddle) + s.tw_off[0];
+  for (int i = threadIdx.x; i < N0; i += blockDim.x) {
+    const float2 w = tw[i];
+    W[i] = make_ulonglong2(pair_const(w.x), pair_const(w.y));
+    xs[i] = -1;
+  }
+  __syncthreads();
+  const int* i0 = s.slab_i0 + k * s.max_slabs;
+  for (int sl = threadIdx.x; sl < s.n_slabs[k]; sl += blockDim.x) {
+    const int x = i0[sl];
+    if (QGB_OK_IDX(x, N0, 63)) xs[x] = sl * s.N[1] * s.N[2];
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ void body_xpass_pair(const qgb_sphere& s, const LocalParams& lp, float2* __restrict__ planes,
+                                                const int b, const int k, const int c0, const int nz) {
+  const int N0 = s.N[0], L1 = s.L1[0], L2 = s.L2[0];
+  const int lim = 32 * N0;
+  cpair_t* sm = smem_pairs();
+  const int* xs = reinterpret_cast<const int*>(sm + lim + N0);
+  const size_t plane = static_cast<size_t>(s.N[1]) * s.N[2];
+  float2* base = planes + plane_index(s, k, b, lp.nb, 0) * plane + c0;
+  const float* V = static_cast<const float*>(s.V) + c0;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
+  const PairLane l{lane, lane < nz, lane + 32 < nz};
+  if (L2 > 1) {
+    xpair_step<0>(L2, base, V, xs, l, plane, L1, L2, lim, lim);
+  } else {
+    for (int x = warp; x < N0; x += nwarps) {
+      const int o = xs[x];
+      sm[x * 32 + lane] = o >= 0 ? pair_load(base + static_cast<unsigned>(o), l) : make_ulonglong2(0, 0);
+    }
+  }
+  __syncthreads();
+  xpair_step<1>(L1, base, V, xs, l, plane, L1, L2, lim, lim);
+  __syncthreads();
+  if (L2 > 1) {
+    xpair_step<2>(L2, base, V, xs, l, plane, L1, L2, lim, lim);
+  } else {
+    for (int x = warp; x < N0; x += nwarps) {
+      const int o = xs[x];
+      const cpair_t v = sm[x * 32 + lane];
+      if (o >= 0) pair_store(base + static_cast<unsigned>(o), l, v.x, v.y);
+    }
+  }
+}
+
 template <typename T>
 __device__ __forceinline__ void body_fft_yz_gather(const qgb_sphere& s, const LocalParams& lp, const cplx_t<T>* C,
                                                    cplx_t<T>* out, const cplx_t<T>* __restrict__ planes,
@@ -588,10 +786,9 @@ __device__ __forceinline__ void body_fft_yz_gather(const qgb_sphere& s, const Lo
 // Kernels: one sphere (grid = work units of that sphere) ...
 // ---------------------------------------------------------------------------
 
-// FP32 takes 80 registers (768 threads an SM), FP64 (block fixed point) 128 (512
-// threads); the CTA sizes follow the grid, see launch_cost.
+// The y/z kernels take 80 registers in FP32 (768 threads an SM), 128 in FP64 (block
+// fixed point, 512 threads); the CTA sizes follow the grid, see launch_cost.
 template <typename T> constexpr int kMaxThreadsYZ = sizeof(T) == 4 ? 384 : 512;
-template <typename T> constexpr int kCtasX = sizeof(T) == 4 ? 3 : 2;
 
 template <typename T>
 __global__ void __launch_bounds__(kMaxThreadsYZ<T>, sizeof(T) == 4 ? 2 : 1) k_ifft_yz(const qgb_sphere s, LocalParams lp,
@@ -600,16 +797,24 @@ __global__ void __launch_bounds__(kMaxThreadsYZ<T>, sizeof(T) == 4 ? 2 : 1) k_if
   body_ifft_yz<T>(s, lp, C, planes, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
-// `tiles` tiles of 32 columns per CTA, one after the other.
-template <typename T>
-__global__ void __launch_bounds__(kThreads, kCtasX<T>) k_xpass(const qgb_sphere s, LocalParams lp,
-                                                            cplx_t<T>* __restrict__ planes, int tiles) {
-  x_tables<T>(s, blockIdx.z, 32 * s.N[0]);
+// `tiles` tiles (x_cols<T> columns: 64 in FP32, 32 in FP64) per CTA, one after the
+// other (one in FP64, whose body a loop costs 4%).
+template <typename T> constexpr int x_cols = sizeof(T) == 4 ? 64 : 32;
+
+template <typename T, int MAXT>
+__global__ void __launch_bounds__(MAXT, MAXT > 160 ? 2 : 4) k_xpass(const qgb_sphere s, LocalParams lp,
+                                                                   cplx_t<T>* __restrict__ planes, int tiles) {
   const int cols = s.N[1] * s.N[2];
-  if (sizeof(T) == 8) tiles = 1;  // (the loop costs FP64 4%)
-  int c0 = blockIdx.x * tiles * 32;
-  for (int t = 0; t < tiles && c0 < cols; ++t, c0 += 32) {
-    if (t > 0) __syncthreads();  // the tile's shared memory is reused
+  if constexpr (sizeof(T) == 4) {
+    x_tables_pair(s, blockIdx.z);
+    int c0 = blockIdx.x * tiles * 64;
+    for (int t = 0; t < tiles && c0 < cols; ++t, c0 += 64) {
+      if (t > 0) __syncthreads();  // the tile's shared memory is reused
+      body_xpass_pair(s, lp, planes, blockIdx.y, blockIdx.z, c0, min(64, cols - c0));
+    }
+  } else {
+    const int c0 = blockIdx.x * 32;
+    x_tables<T>(s, blockIdx.z, 32 * s.N[0]);
     body_xpass<T, true>(s, lp, planes, blockIdx.y, blockIdx.z, c0, min(32, cols - c0));
   }
 }
@@ -636,11 +841,10 @@ inline size_t x_smem_bytes(const qgb_sphere& s, int nz, size_t e) {
 constexpr size_t kSmemPerSm = 227 * 1024;
 
 // Relative cost of a launch: `ctas_total` CTAs of t threads and `smem` bytes,
-// each doing `work` thread-rounds (a round counts its codelet's elements).  An
-// SM holds 768 threads of 80 registers in FP32, 512 of 128 in FP64; wide CTAs
-// wait longer at their barriers; a launch of few CTAs takes whole waves.
-template <typename T> double launch_cost(double ctas_total, int t, size_t smem, double work) {
-  const int resident = sizeof(T) == 4 ? 768 : 512;
+// each doing `work` thread-rounds (a round counts its codelet's elements), where
+// an SM's registers hold `resident` threads.  Wide CTAs wait longer at their
+// barriers; a launch of few CTAs takes whole waves.
+inline double launch_cost(int resident, double ctas_total, int t, size_t smem, double work) {
   const int ctas = std::max(1, static_cast<int>(std::min<size_t>(resident / t, (kSmemPerSm + 1024) / (smem + 1024))));
   double waves = std::max(1.0, ctas_total / (152.0 * ctas));
   if (waves < 8.0) waves = std::ceil(waves);
@@ -661,7 +865,7 @@ template <typename T> int threads_yz(const qgb_sphere& s, int nb) {
     auto rounds = [t](int items) { return (items + t - 1) / t; };
     const double work = rounds(s.N[2] * s.L1[1]) * s.L2[1] + rounds(s.N[2] * s.L2[1]) * s.L1[1] +
                         rounds(zrows * s.L1[2]) * s.L2[2] + rounds(zrows * s.L2[2]) * s.L1[2] + 8.0;
-    const double cost = launch_cost<T>(static_cast<double>(s.max_slabs) * nb * s.nk, t, smem, work);
+    const double cost = launch_cost(sizeof(T) == 4 ? 768 : 512, static_cast<double>(s.max_slabs) * nb * s.nk, t, smem, work);
     if (cost < best * 0.999) {
       best = cost;
       threads = t;
@@ -670,32 +874,54 @@ template <typename T> int threads_yz(const qgb_sphere& s, int nb) {
   return threads;
 }
 
+// CTAs of the FP32 x-pass of up to 160 threads have 96 registers, four an SM, while
+// shared memory lets three in (N0 <= 136); longer axes take up to 256 threads of
+// 128 registers.  FP64 takes the latter always.  (96^3, 160 bands / 72^3, 800
+// bands, us: 160 threads 367 / 774, 192 of 112 registers 354 / 842, 256 360 / 843.)
+template <typename T> int x_max_threads(size_t smem) {
+  return sizeof(T) == 4 && 3 * (smem + 1024) <= kSmemPerSm + 1024 ? 160 : kThreads;
+}
+
 // CTA size of the x-pass and the tiles a CTA takes.  A plane's N1 N2 columns are
-// one contiguous range, so its tiles need not be y-rows: they are 32 columns
-// (256 B of a row in FP32), and the warps take the L1 subs of the outer passes
+// one contiguous range, so its tiles need not be y-rows: they are x_cols columns
+// (512 B of a row), and the warps take the L1 subs of the outer passes
 // (radix L2, twice) and the L2 of the middle step (radix L1, both directions) in
 // as few rounds as launch_cost allows.  si64 (96^3): 3 + 2 full rounds of 4 warps.
 // In FP32 up to 8 tiles share a CTA's tables while 4 waves of CTAs are left.
 // Measured against whole y-rows flattened over 256 threads (x-pass, us): si64, 160
-// bands 436 -> 377 (FP64, 32 bands 592 -> 568), 36^3, 144 bands 38 -> 21 (FP64 177 ->
-// 136), 72^3, 800 bands 1046 -> 862.
+// bands 436 -> 367 (FP64, 32 bands 592 -> 568), 36^3, 144 bands 38 -> 20 (FP64 177 ->
+// 136), 72^3, 800 bands 1046 -> 751.
 template <typename T> void x_shape(const qgb_sphere& s, int nb, int* threads, int* tiles) {
   const int L1 = s.L1[0], L2 = s.L2[0];
-  const size_t smem = x_smem_bytes(s, 32, sizeof(cplx_t<T>));
-  const double total = (static_cast<double>(s.N[1]) * s.N[2] + 31) / 32 * nb * s.nk;
+  const size_t smem = x_smem_bytes(s, 32, 16);
+  const int max_threads = x_max_threads<T>(smem), resident = max_threads == 160 ? 640 : 512;
+  const double total = (static_cast<double>(s.N[1]) * s.N[2] + x_cols<T> - 1) / x_cols<T> * nb * s.nk;
   double best = 1e30;
   *threads = 128;
-  for (int w = 1; w <= kThreads / 32; ++w) {
+  for (int w = 1; w <= max_threads / 32; ++w) {
     const int outer = L2 > 1 ? (L1 + w - 1) / w : 0, mid = (L2 + w - 1) / w;
     const double work = 2.0 * (outer * L2 + mid * L1) + 8.0;
-    const double cost = launch_cost<T>(total, 32 * w, smem, work);
+    const double cost = launch_cost(resident, total, 32 * w, smem, work);
     if (cost < best * 0.999) {
       best = cost;
       *threads = 32 * w;
     }
   }
-  const int ctas = std::max(1, (sizeof(T) == 4 ? 768 : 512) / *threads);
+  const int ctas = std::max(1, resident / *threads);
   *tiles = sizeof(T) == 8 ? 1 : std::max(1, std::min(8, static_cast<int>(total / (4.0 * 152.0 * ctas))));
+}
+
+template <typename T, int MAXT>
+int launch_x(const qgb_sphere& s, const LocalParams& lp, void* planes, cudaStream_t st) {
+  const size_t smem = x_smem_bytes(s, 32, 16);  // rows of 32 x 16 B: double complex, or two of float
+  if (int rc = raise_smem_limit(k_xpass<T, MAXT>, smem)) return rc;
+  int threads, tiles;
+  x_shape<T>(s, lp.nb, &threads, &tiles);
+  const int cta_cols = x_cols<T> * tiles;
+  k_xpass<T, MAXT><<<dim3((s.N[1] * s.N[2] + cta_cols - 1) / cta_cols, lp.nb, s.nk), threads, smem, st>>>(
+      s, lp, static_cast<cplx_t<T>*>(planes), tiles);
+  QGB_LAUNCH_CHECK("k_xpass");
+  return QGB_OK;
 }
 
 template <typename T>
@@ -714,13 +940,13 @@ int launch_chunk(const qgb_sphere& s, const LocalParams& lp, const void* C, void
   using C2 = cplx_t<T>;
   int rc;
   if ((rc = launch_ifft_yz<T>(s, lp, C, planes, st))) return rc;
-  const size_t smx = x_smem_bytes(s, 32, sizeof(C2));
-  if ((rc = raise_smem_limit(k_xpass<T>, smx))) return rc;
-  int tx, tiles;
-  x_shape<T>(s, lp.nb, &tx, &tiles);
-  k_xpass<T><<<dim3((s.N[1] * s.N[2] + 32 * tiles - 1) / (32 * tiles), lp.nb, s.nk), tx, smx, st>>>(
-      s, lp, static_cast<C2*>(planes), tiles);
-  QGB_LAUNCH_CHECK("k_xpass");
+  if constexpr (sizeof(T) == 4) {
+    rc = x_max_threads<T>(x_smem_bytes(s, 32, 16)) == 160 ? launch_x<T, 160>(s, lp, planes, st)
+                                                          : launch_x<T, kThreads>(s, lp, planes, st);
+  } else {
+    rc = launch_x<T, kThreads>(s, lp, planes, st);
+  }
+  if (rc) return rc;
   if (gather_after) QGB_CUDA_CHECK(cudaStreamWaitEvent(st, gather_after, 0));
   const size_t smem = yz_smem_bytes(s, sizeof(C2));
   if ((rc = raise_smem_limit(k_fft_yz_gather<T>, smem))) return rc;
