@@ -14,9 +14,10 @@
 //                  an N1 x N2 plane in shared memory, inverse z-FFT on the rows
 //                  the sphere touches, inverse y-FFT on all columns, store the
 //                  plane (real-space y, z in permuted order) to the workspace.
-//   k_xpass        one CTA per (k, band, y-row): gather the slabs' rows into
-//                  N2 pencils along x, inverse x-FFT, multiply by V(r), forward
-//                  x-FFT, keep only the slab rows, store back.
+//   k_xpass        one CTA per (k, band, tiles of 64 (FP32) or 32 (FP64) of the
+//                  plane's columns): gather the slabs' rows into pencils along
+//                  x, inverse x-FFT, multiply by V(r), forward x-FFT, keep only
+//                  the slab rows, store back.
 //   k_fft_yz_gather one CTA per (k, band, slab): forward y-FFT on all columns,
 //                  forward z-FFT on the touched rows, gather the slab's points,
 //                  scale by 1/N and add KE*psi.

@@ -6,13 +6,17 @@
 // pairs of columns halve the arithmetic's share of the issue slots and the
 // addressing around it.  Each half is rounded like the scalar operation.
 //
-// F2 is the codelets' type T: a pair with a pending sign and a pending constant
-// factor, both known at compile time once a codelet is unrolled, which fold into
-// the next addition (subtraction, multiply-add) as the compiler folds them for
-// float.
+// Lazy<L> is the codelets' type T: a pair (L = pair_t) with a pending sign and a
+// pending constant factor, both known at compile time once a codelet is unrolled,
+// which fold into the next addition (subtraction, multiply-add) as the compiler
+// folds them for float.  Lazy<float> does the same operations on one column: the
+// batched x-pass, which takes y-rows, gives the same bits.
 #pragma once
 
 #include <cstdint>
+
+#include "block_fixed.cuh"
+#include "codelets.cuh"
 
 namespace qgb {
 
@@ -28,99 +32,135 @@ __device__ __forceinline__ float2 pair_split(pair_t v) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
   return r;
 }
-__device__ __forceinline__ pair_t pair_add(pair_t a, pair_t b) {
+__device__ __forceinline__ pair_t lane_add(pair_t a, pair_t b) {
   pair_t r;
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
-__device__ __forceinline__ pair_t pair_mul(pair_t a, pair_t b) {
+__device__ __forceinline__ pair_t lane_mul(pair_t a, pair_t b) {
   pair_t r;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
-__device__ __forceinline__ pair_t pair_fma(pair_t a, pair_t b, pair_t c) {
+__device__ __forceinline__ pair_t lane_fma(pair_t a, pair_t b, pair_t c) {
   pair_t r;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
-__device__ __forceinline__ pair_t pair_const(float c) { return pair_of(c, c); }
+__device__ __forceinline__ pair_t lane_neg(pair_t a) { return a ^ 0x8000000080000000ull; }
+__device__ __forceinline__ float lane_add(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float lane_mul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float lane_fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ float lane_neg(float a) { return -a; }
+template <typename L> __device__ __forceinline__ L lane_const(float c) {
+  if constexpr (sizeof(L) == 8)
+    return pair_of(c, c);
+  else
+    return c;
+}
 
-struct F2 {
-  pair_t v = 0;
+template <typename L> struct Lazy {
+  L v = 0;
   float c = 1.0f;        // the value is +-c v; c alone for a literal
   bool neg = false, scaled = false, literal = false;
-  F2() = default;
-  __device__ __forceinline__ explicit F2(double x) : c(static_cast<float>(x)), literal(true) {}
-  __device__ __forceinline__ static F2 of(pair_t p) {
-    F2 r;
+  Lazy() = default;
+  __device__ __forceinline__ explicit Lazy(double x) : c(static_cast<float>(x)), literal(true) {}
+  __device__ __forceinline__ static Lazy of(L p) {
+    Lazy r;
     r.v = p;
     return r;
   }
-  __device__ __forceinline__ pair_t value() const {
-    if (scaled) return pair_mul(v, pair_const(neg ? -c : c));
-    return neg ? pair_mul(v, pair_const(-1.0f)) : v;
+  __device__ __forceinline__ L value() const {
+    if (scaled) return lane_mul(v, lane_const<L>(neg ? -c : c));
+    return neg ? lane_mul(v, lane_const<L>(-1.0f)) : v;
   }
 };
 
-__device__ __forceinline__ F2 operator-(F2 a) {
+template <typename L> __device__ __forceinline__ Lazy<L> operator-(Lazy<L> a) {
   a.neg = !a.neg;
   return a;
 }
 
 // Literal times pair: left pending, or a product of its own on a pending one.
-__device__ __forceinline__ F2 operator*(const F2& l, const F2& a) {
-  F2 r;
-  r.v = a.scaled ? pair_mul(a.v, pair_const(a.c)) : a.v;
+template <typename L> __device__ __forceinline__ Lazy<L> operator*(const Lazy<L>& l, const Lazy<L>& a) {
+  Lazy<L> r;
+  r.v = a.scaled ? lane_mul(a.v, lane_const<L>(a.c)) : a.v;
   r.neg = a.neg;
   r.c = l.c;
   r.scaled = true;
   return r;
 }
 
-__device__ __forceinline__ F2 operator+(const F2& a, const F2& b) {
-  F2 r;
+template <typename L> __device__ __forceinline__ Lazy<L> operator+(const Lazy<L>& a, const Lazy<L>& b) {
+  Lazy<L> r;
   if (b.scaled) {
     // b's factor takes the sign relative to a's base.
-    pair_t base = a.v;
+    L base = a.v;
     bool base_neg = a.neg;
     if (a.scaled) {
-      base = pair_mul(a.v, pair_const(a.neg ? -a.c : a.c));
+      base = lane_mul(a.v, lane_const<L>(a.neg ? -a.c : a.c));
       base_neg = false;
     }
-    r.v = pair_fma(b.v, pair_const(b.neg != base_neg ? -b.c : b.c), base);
+    r.v = lane_fma(b.v, lane_const<L>(b.neg != base_neg ? -b.c : b.c), base);
     r.neg = base_neg;
   } else if (a.scaled) {
-    r.v = pair_fma(a.v, pair_const(a.neg != b.neg ? -a.c : a.c), b.v);
+    r.v = lane_fma(a.v, lane_const<L>(a.neg != b.neg ? -a.c : a.c), b.v);
     r.neg = b.neg;
   } else if (a.neg == b.neg) {
-    r.v = pair_add(a.v, b.v);
+    r.v = lane_add(a.v, b.v);
     r.neg = a.neg;
   } else if (b.neg) {
-    r.v = pair_fma(b.v, pair_const(-1.0f), a.v);
+    r.v = lane_fma(b.v, lane_const<L>(-1.0f), a.v);
   } else {
-    r.v = pair_fma(a.v, pair_const(-1.0f), b.v);
+    r.v = lane_fma(a.v, lane_const<L>(-1.0f), b.v);
   }
   return r;
 }
-__device__ __forceinline__ F2 operator-(const F2& a, const F2& b) { return a + (-b); }
+template <typename L> __device__ __forceinline__ Lazy<L> operator-(const Lazy<L>& a, const Lazy<L>& b) { return a + (-b); }
+using F2 = Lazy<pair_t>;
 
 // A complex pair in shared memory: 16 B, (re, im) of both columns.
 using cpair_t = ulonglong2;
 
-// The codelet block of pairs; see Block<float, R>.
-template <int R> struct PairBlock {
-  F2 re[R], im[R];
+// The codelet block of either; see Block<float, R>.  The twiddles w.x, w.y are of
+// the lanes' type (doubled for pairs).
+template <typename L, int R> struct LazyBlock {
+  Lazy<L> re[R], im[R];
   template <int S> __device__ __forceinline__ void run() { Codelet<R, S>::run(re, im); }
-  // Element j times (w.x, w.y), both already doubled to pairs (S < 0: its conjugate).
-  template <int S> __device__ __forceinline__ void twiddle(int j, cpair_t w) {
-    const pair_t x = re[j].value(), y = im[j].value();
-    const pair_t wy = S > 0 ? w.y : w.y ^ 0x8000000080000000ull, wn = S > 0 ? w.y ^ 0x8000000080000000ull : w.y;
-    re[j] = F2::of(pair_fma(y, wn, pair_mul(x, w.x)));
-    im[j] = F2::of(pair_fma(x, wy, pair_mul(y, w.x)));
+  // Element j times (wx, wy) (S < 0: its conjugate).
+  template <int S> __device__ __forceinline__ void twiddle(int j, L wx, L wy) {
+    const L x = re[j].value(), y = im[j].value();
+    const L wp = S > 0 ? wy : lane_neg(wy), wn = S > 0 ? lane_neg(wy) : wy;
+    re[j] = Lazy<L>::of(lane_fma(y, wn, lane_mul(x, wx)));
+    im[j] = Lazy<L>::of(lane_fma(x, wp, lane_mul(y, wx)));
   }
-  __device__ __forceinline__ void scale(int j, pair_t f) {
-    re[j] = F2::of(pair_mul(re[j].value(), f));
-    im[j] = F2::of(pair_mul(im[j].value(), f));
+  __device__ __forceinline__ void scale(int j, L f) {
+    re[j] = Lazy<L>::of(lane_mul(re[j].value(), f));
+    im[j] = Lazy<L>::of(lane_mul(im[j].value(), f));
+  }
+};
+template <int R> using PairBlock = LazyBlock<pair_t, R>;
+
+// The x-pass's block on one column: Block<T, R>, in FP32 with the pairs' operations.
+template <typename T, int R> struct XBlock : Block<T, R> {};
+template <int R> struct XBlock<float, R> {
+  LazyBlock<float, R> x;
+  __device__ __forceinline__ void load(const float (&re)[R], const float (&im)[R]) {
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+      x.re[j] = Lazy<float>::of(re[j]);
+      x.im[j] = Lazy<float>::of(im[j]);
+    }
+  }
+  template <int S> __device__ __forceinline__ void run() { x.template run<S>(); }
+  template <int S> __device__ __forceinline__ void twiddle(int j, float2 w) { x.template twiddle<S>(j, w.x, w.y); }
+  __device__ __forceinline__ void scale(const float (&v)[R]) {
+#pragma unroll
+    for (int j = 0; j < R; ++j) x.scale(j, v[j]);
+  }
+  template <typename F> __device__ __forceinline__ void store(F put) const {
+#pragma unroll
+    for (int j = 0; j < R; ++j) put(j, [&] { return make_float2(x.re[j].value(), x.im[j].value()); });
   }
 };
 
