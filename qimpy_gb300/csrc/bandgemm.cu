@@ -551,6 +551,9 @@ int gram(int dtype, int out_dtype, const void* A, long long a_batch, int lda, co
   if (out_dtype != QGB_F64 && out_dtype != QGB_F32) return fail(QGB_ERR_INVALID, "unknown out dtype %d", out_dtype);
   if (dtype == QGB_F64 && out_dtype == QGB_F32) return fail(QGB_ERR_UNSUPPORTED, "FP64 gram to FP32 output");
   if (K == 0) return fail(QGB_ERR_INVALID, "gram over an empty basis");
+  const GramPlan p = gram_plan(nk, M, N, K, elem_bytes(dtype));
+  if (p.splits > 1 && (!ws || ws_bytes < p.partial_bytes))
+    return fail(QGB_ERR_WORKSPACE, "gram workspace %zu B < %zu B", ws_bytes, p.partial_bytes);
   if (dtype == QGB_F64 && ws && oz_gram_use(nk, M, N, K) &&
       ws_bytes >= oz_gram_workspace_bytes(nk, M, N, K, real_out))
     return oz_gram(A, a_batch, lda, B, b_batch, ldb, nk, M, N, K, out, out_batch, oi, oj, ws, st, weight, real_out);
@@ -566,9 +569,6 @@ int gram(int dtype, int out_dtype, const void* A, long long a_batch, int lda, co
     QGB_LAUNCH_CHECK("k_gram_small");
     return QGB_OK;
   }
-  const GramPlan p = gram_plan(nk, M, N, K, elem_bytes(dtype));
-  if (p.splits > 1 && (!ws || ws_bytes < p.partial_bytes))
-    return fail(QGB_ERR_WORKSPACE, "gram workspace %zu B < %zu B", ws_bytes, p.partial_bytes);
   GramArgs g{A, B, a_batch, b_batch, lda, ldb, M, N, K, p.splits, p.g_per_split, ws, out, out_batch, oi, oj,
              weight, real_out ? 1 : 0};
   const dim3 grid(p.ti, p.tj, nk * p.splits);

@@ -102,3 +102,21 @@ def test_back_projection(nk, atoms, pa, nb, G, dtype):
     want = oh + np.einsum("kpg,kbp->kbg", bh, Dp)
     mag = np.abs(oh) + np.einsum("kpg,kbp->kbg", np.abs(bh), Dm)
     assert np.all(np.abs(got - want) <= _bound(P + pa + 1, dtype, mag))
+
+
+def test_short_workspace_is_refused():
+    """The overlap's workspace is asked for on every route, also where the small kernel has no use for it."""
+    from qimpy_gb300 import _lib
+
+    lib = _lib.lib()
+    X = torch.ones((1, 8, 4000), dtype=torch.complex128, device=DEV)
+    out = torch.empty((1, 8, 8), dtype=torch.complex128, device=DEV)
+    need = lib.qgb_dot_workspace_bytes(_lib.QGB_F64, 1, 8, 8, 4000)
+    assert need > 0
+    ws = torch.empty(need, dtype=torch.uint8, device=DEV)
+    st = torch.cuda.current_stream().cuda_stream
+    args = (_lib.QGB_F64, X.data_ptr(), 8, X.data_ptr(), 8, 1, 4000, out.data_ptr())
+    assert lib.qgb_dot(*args, None, 0, st) != 0
+    assert lib.qgb_dot(*args, ws.data_ptr(), need - 1, st) != 0
+    assert lib.qgb_dot(*args, ws.data_ptr(), need, st) == 0
+    assert torch.equal(out, torch.full_like(out, 4000.0))
