@@ -292,7 +292,7 @@ def local_roofline(rc, band_apps, t_loc, hbm_peak, peaks) -> dict:
     ach_tflops = rc["flops_loc"] * band_apps / t_loc / 1e12
     traffic = NCU_DRAM_BYTES_PER_BLOCK["local"]
     t_lb = max(rc["bytes_loc"] * band_apps / (hbm_peak * 1e9), rc["flops_loc"] * band_apps / (peaks["fp32"] * 1e12))
-    return {"kernel": "local potential: k_ifft_yz + k_xpass_async + k_fft_yz_gather, one 32-band block, FP32",
+    return {"kernel": "local potential: k_ifft_yz + k_xpass + k_fft_yz_gather, one 32-band block, FP32",
             "bound": "hbm", "achieved": ach_gbs, "peak": hbm_peak, "unit": "GB/s", "frac": ach_gbs / hbm_peak,
             "peak_source": "measured (MEASURED_PEAKS.json hbm_gbs)", "traffic": traffic,
             "traffic_source": "constant: one cold-cache ncu capture of a 32-band block",
@@ -531,7 +531,7 @@ def run_gb300(args, rank, ws, local):
         # our kernels per step: 3 local-potential kernels per FFT block, plus the
         # nonlocal term once per call: 5 tensor-core chain kernels (mixed) or the
         # Gram, its reduction, D and the rotation (FP64)
-        res["launches_per_step"] = 3 * len(blocks) + (5 if mixed else 4) * (1 if one_call else len(blocks))
+        res["launches_per_step"] = 3 * len(blocks) + (5 if mixed else 13) * (1 if one_call else len(blocks))
         res["nonlocal_error_word"] = int(ops.device_error_word(dev).item()) if mixed else 0
         res["real_bytes"] = 8 if cdt == torch.complex128 else 4
         res["fft_schedule"] = [list(f) for f in ds.tables.fac]
