@@ -807,8 +807,8 @@ __device__ __forceinline__ void body_fft_yz_gather(const qgb_sphere& s, const Lo
       const C2 f = sm[pos];
       T xr = f.x * invN, xi = f.y * invN;
       if (add_ke) {
-        xr = e[u] * c[u].x + xr;
-        xi = e[u] * c[u].y + xi;
+        xr = fma(e[u], c[u].x, xr);  // (KE, the larger term at high G, unrounded)
+        xi = fma(e[u], c[u].y, xi);
       }
       if (accumulate) {
         xr += o[u].x;
