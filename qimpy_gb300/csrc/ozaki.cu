@@ -31,6 +31,7 @@
 // Kernels (for each complex product as real ones: rows Re and Im stacked, or
 // folded along K where only the real part is kept):
 //   k_oz_slice_rows   A and B of an overlap: K-contiguous rows -> digits
+//   k_oz_band_exp     a rotation's bands: their scales
 //   k_oz_slice_cols   X of a rotation (contracted over its rows): transposed
 //   k_oz_slice_mat    W of a rotation
 //   k_oz_gemm         tcgen05 GEMM over digits, 128 x 64 outputs per CTA
@@ -68,7 +69,9 @@ constexpr int SUMS_OFF = BAR_OFF + 512;
 constexpr int SMEM_BYTES = SUMS_OFF + EPI_WARPS * 2 * SUMS_LD * 16 + 1024;
 static_assert((2 * S + 6 + 2 * ND + 1) * 8 + 16 <= 512 && SMEM_BYTES <= 227 * 1024, "shared memory layout");
 constexpr int kThreads = (EPI_WARPS + 2) * 32;
-constexpr int kNonFinite = 0x7FF;  // exponent mark of rows with a NaN or an infinity
+constexpr int kNonFinite = 0x7FF;  // exponent mark of an overlap's rows with a NaN or an infinity
+constexpr int kBadRow = 1 << 16;   // the same mark of a rotation's rows, whose exponents go up to 2 * 2046
+constexpr int kNoEntry = -4096;    // exponent of a rotation's row without a nonzero entry
 
 enum Epi { EPI_PARTIAL = 0, EPI_ROTATE = 1 };
 
@@ -391,7 +394,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             double2 v;
             if (!ok) {
               v = make_double2(nan, nan);
-            } else if (eg == kNonFinite || ew[j] == kNonFinite) {
+            } else if (eg == kBadRow || ew[j] == kBadRow) {
               const double2* x = args.X + t.batch * args.x_batch + g;
               const double2* wp = args.W + t.batch * args.w_batch + static_cast<long long>(j) * args.wj;
               v = make_double2(0.0, 0.0);
@@ -437,15 +440,25 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 __device__ __forceinline__ int exp_field(double x) { return (__double2hiint(x) >> 20) & 0x7FF; }
 
+// Largest exponent field of a complex number, 1 if that is subnormal and 0 only
+// for zero.  By integers: comparing doubles would take the FP64 pipe.
+__device__ __forceinline__ int scale_field(double2 v) {
+  const unsigned hi = max(static_cast<unsigned>(__double2hiint(v.x)) & 0x7FFFFFFFu,
+                          static_cast<unsigned>(__double2hiint(v.y)) & 0x7FFFFFFFu);
+  const unsigned any = hi | static_cast<unsigned>(__double2loint(v.x)) | static_cast<unsigned>(__double2loint(v.y));
+  return static_cast<int>(max(hi >> 20, min(any, 1u)));
+}
+
 // round(x 2^(54 - (emax - 1023))) for |x| of exponent field at most emax: below
-// 2^55 in magnitude, exact for the values within 2 bits of the largest.
+// 2^55 in magnitude, exact for the values within 2 bits of the largest.  Zero
+// gives zero for any emax.
 __device__ __forceinline__ long long fixed_point(double x, int emax) {
   const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(x));
   int E = static_cast<int>(b >> 52) & 0x7FF;
   unsigned long long m = b & 0x000FFFFFFFFFFFFFull;
   if (E > 0) m |= 0x0010000000000000ull; else E = 1;
   const int sh = emax - E - 2;
-  const long long X = static_cast<long long>(sh <= 0 ? m << (-sh) : (sh > 54 ? 0ull : (m + (1ull << (sh - 1))) >> sh));
+  const long long X = static_cast<long long>(sh <= 0 ? m << (-sh & 3) : (sh > 54 ? 0ull : (m + (1ull << (sh - 1))) >> sh));
   return static_cast<long long>(b) < 0 ? -X : X;
 }
 
@@ -547,32 +560,67 @@ __global__ void __launch_bounds__(256) k_oz_slice_rows(const SliceArgs a0, const
   }
 }
 
+// The contracted index of a rotation is the band, and bands may differ by any
+// factor (unnormalised ones, filtered ones, projectors of a back-projection): a
+// common exponent would cut the small ones off.  So band i is scaled by its own
+// power of two, s_i = 2^(e_i - 1023) with e_i the largest exponent field of its
+// finite entries, and the product is of X_i / s_i and s_i W(i, j).  Both are
+// shifts of the exponents the slices are taken at, exact, and cancel in the
+// result.  A CTA takes kExpRange g of a band, all loads in flight: 39 us for
+// 352 x 37073, of which the read takes 31 (ranges four times as long, in a loop: 44).
+constexpr int kExpRange = 2048;
+__global__ void __launch_bounds__(256) k_oz_band_exp(const double2* __restrict__ X, long long x_batch, int ldx, int Kin,
+                                                     int G, int* __restrict__ e) {
+  __shared__ int red[8];
+  const int i = blockIdx.x, batch = blockIdx.z, g0 = blockIdx.y * kExpRange + threadIdx.x;
+  const double2* x = X + batch * x_batch + static_cast<long long>(i) * ldx;
+  double2 v[kExpRange / 256];
+#pragma unroll
+  for (int u = 0; u < kExpRange / 256; ++u) {
+    const int g = g0 + 256 * u;
+    v[u] = g < G ? x[g] : make_double2(0.0, 0.0);
+  }
+  int em = 0;
+#pragma unroll
+  for (int u = 0; u < kExpRange / 256; ++u) {
+    // (an entry with a non-finite part counts by neither part: its row is marked)
+    const int f = scale_field(v[u]);
+    em = max(em, f == kNonFinite ? 0 : f);
+  }
+  em = block_max<256>(em, red);
+  if (threadIdx.x == 0) atomicMax(e + static_cast<long long>(batch) * Kin + i, em);  // zero before the launch
+}
+
 // X [batch][Kin][ldx] of a rotation -> digits [batch][7][rows][ld], row = g,
-// K = [Re X_i, i < Kh | Im X_i], one exponent per g.  One CTA per 32 g: pass 1
-// takes the exponents, pass 2 transposes 32 x 32 tiles through shared memory.
+// K = [Re X_i, i < Kh | Im X_i], one exponent per g, of the scaled bands.  One CTA
+// per 32 g: pass 1 takes the exponents, pass 2 transposes 32 x 32 tiles through
+// shared memory.
 __global__ void __launch_bounds__(256) k_oz_slice_cols(const double2* __restrict__ X, long long x_batch, int ldx,
                                                        int Kin, int Kh, int g0, int G, int rows,
                                                        __nv_bfloat16* __restrict__ digits, int ld,
-                                                       int* __restrict__ e, int* err) {
+                                                       const int* __restrict__ eband, int* __restrict__ e, int* err) {
   __shared__ double2 tile[32][33];
-  __shared__ int red[8][32];
+  __shared__ int red[8][32], tile_e[32];
   if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && err) *err = 0;
   const int batch = blockIdx.y, r0 = blockIdx.x * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int g = g0 + r0 + tx;
   const bool gin = r0 + tx < rows && g < G;
   const double2* x = X + batch * x_batch + g;
-  int em = 1;
+  const int* eb = eband + static_cast<long long>(batch) * Kin;
+  int em = kNoEntry;
   if (gin)
+#pragma unroll 4
     for (int i = ty; i < Kin; i += 8) {
-      const double2 v = x[static_cast<long long>(i) * ldx];
-      em = max(em, max(exp_field(v.x), exp_field(v.y)));
+      const int f = scale_field(x[static_cast<long long>(i) * ldx]);
+      em = max(em, f > 0 ? f - eb[i] : kNoEntry);  // above 0 only where f is kNonFinite
     }
   red[ty][tx] = em;
   __syncthreads();
   if (ty == 0) {
 #pragma unroll
     for (int w = 1; w < 8; ++w) em = max(em, red[w][tx]);
+    if (em > 0) em = kBadRow;
     red[0][tx] = em;
     if (gin) e[static_cast<long long>(batch) * rows + r0 + tx] = em;
   }
@@ -587,15 +635,16 @@ __global__ void __launch_bounds__(256) k_oz_slice_cols(const double2* __restrict
       const int i = i0 + ty + 8 * w;
       tile[ty + 8 * w][tx] = (gin && i < Kin) ? x[static_cast<long long>(i) * ldx] : make_double2(0.0, 0.0);
     }
+    if (ty == 0) tile_e[tx] = i0 + tx < Kin ? eb[i0 + tx] : 0;
     __syncthreads();
     if (r0 + rr < rows && i0 + seg < Kh) {
       unsigned long long re[4], im[4];
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
         double2 v = tile[seg + t][rr];
-        if (er == kNonFinite) v = make_double2(0.0, 0.0);
-        re[t] = biased_digits(v.x, er);
-        im[t] = biased_digits(v.y, er);
+        if (er == kBadRow) v = make_double2(0.0, 0.0);
+        re[t] = biased_digits(v.x, er + tile_e[seg + t]);
+        im[t] = biased_digits(v.y, er + tile_e[seg + t]);
       }
       store_digits4(dst + i0 + seg, step, re);
       store_digits4(dst + Kh + i0 + seg, step, im);
@@ -607,19 +656,22 @@ __global__ void __launch_bounds__(256) k_oz_slice_cols(const double2* __restrict
 // W(i, j) of a rotation -> digits of real rows [batch][7][2 * Npad][ld]: column
 // tile t of 64 rows holds bands 32 t + 8 h + jj (h < 4, jj < 8) as rows
 // 64 t + 16 h + jj (real output: Re W, -Im W) and + 8 (imaginary: Im W, Re W),
-// so one epilogue warp has both parts of its bands.  One CTA per band.
+// so one epilogue warp has both parts of its bands.  One CTA per band.  Row i is
+// scaled by the power of two of band i of X (a band of zeros adds nothing).
 __global__ void __launch_bounds__(128) k_oz_slice_mat(const double2* __restrict__ W, long long w_batch, int wi, int wj,
                                                       int Kin, int Kh, int Nout, int Npad,
                                                       __nv_bfloat16* __restrict__ digits, int ld,
-                                                      int* __restrict__ e) {
+                                                      const int* __restrict__ eband, int* __restrict__ e) {
   __shared__ int red[4];
   const int j = blockIdx.x, batch = blockIdx.y;
   const double2* w = W + batch * w_batch + static_cast<long long>(j) * wj;
-  int em = 1;
+  const int* eb = eband + static_cast<long long>(batch) * Kin;
+  int em = kNoEntry;
   if (j < Nout)
     for (int i = threadIdx.x; i < Kin; i += 128) {
       const double2 v = w[static_cast<long long>(i) * wi];
-      em = max(em, max(exp_field(v.x), exp_field(v.y)));
+      const int f = scale_field(v);
+      em = max(em, f == kNonFinite ? kBadRow : (f > 0 && eb[i] > 0 ? f + eb[i] : kNoEntry));
     }
   em = block_max<128>(em, red);
   if (threadIdx.x == 0) e[static_cast<long long>(batch) * Npad + j] = em;
@@ -632,10 +684,11 @@ __global__ void __launch_bounds__(128) k_oz_slice_mat(const double2* __restrict_
 #pragma unroll
     for (int t = 0; t < 4; ++t) {
       double2 v = make_double2(0.0, 0.0);
-      if (j < Nout && i + t < Kin && em != kNonFinite) v = w[static_cast<long long>(i + t) * wi];
-      re[t] = biased_digits(v.x, em);
-      im[t] = biased_digits(v.y, em);
-      mi[t] = biased_digits(-v.y, em);
+      const int ei = i + t < Kin ? eb[i + t] : 0;
+      if (j < Nout && ei > 0 && em != kBadRow) v = w[static_cast<long long>(i + t) * wi];
+      re[t] = biased_digits(v.x, em - ei);
+      im[t] = biased_digits(v.y, em - ei);
+      mi[t] = biased_digits(-v.y, em - ei);
     }
     store_digits4(dre + i, step, re);
     store_digits4(dre + Kh + i, step, mi);
@@ -831,7 +884,7 @@ static OzRot rot_layout(int nk, int Kin, int Nout, int G) {
   L.panels = (G + L.rows - 1) / L.rows;
   L.a_elems = round_up(nk * S * static_cast<long long>(L.rows) * L.ld, 128);
   L.b_elems = round_up(nk * S * 2ll * L.Npad * L.ld, 128);
-  L.e_bytes = static_cast<size_t>(round_up(static_cast<long long>(nk) * (L.rows + L.Npad) * 4, 256));
+  L.e_bytes = static_cast<size_t>(round_up(static_cast<long long>(nk) * (L.rows + L.Npad + Kin) * 4, 256));
   L.total = static_cast<size_t>(L.a_elems + L.b_elems) * 2 + L.e_bytes + 256 + 256;
   return L;
 }
@@ -851,7 +904,8 @@ bool oz_gram_use(int nk, int M, int N, int K) {
   return oz_worth(static_cast<double>(nk) * M * N * K) && nk <= 4096 && M <= 65535 && N <= 65535;
 }
 bool oz_rotate_use(int nk, int Kin, int Nout, int G) {
-  return oz_worth(static_cast<double>(nk) * Kin * Nout * G) && nk <= 4096 && Nout <= 65535;
+  return oz_worth(static_cast<double>(nk) * Kin * Nout * G) && nk <= 4096 && Nout <= 65535 &&
+         G <= 65535 * kExpRange;
 }
 
 size_t oz_gram_workspace_bytes(int nk, int M, int N, int K, bool real_out) {
@@ -922,15 +976,21 @@ int oz_rotate(const void* X, long long x_batch, int ldx, const void* W, long lon
   p += (L.a_elems + L.b_elems) * 2;
   int* eg = reinterpret_cast<int*>(p);
   int* ew = eg + static_cast<long long>(nk) * L.rows;
+  int* eb = ew + static_cast<long long>(nk) * L.Npad;
+  QGB_CUDA_CHECK(cudaMemsetAsync(eb, 0, static_cast<size_t>(nk) * Kin * sizeof(int), st));
+  k_oz_band_exp<<<dim3(Kin, (G + kExpRange - 1) / kExpRange, nk), 256, 0, st>>>(static_cast<const double2*>(X), x_batch,
+                                                                                ldx, Kin, G, eb);
+  QGB_LAUNCH_CHECK("k_oz_band_exp");
   k_oz_slice_mat<<<dim3(L.Npad, nk), 128, 0, st>>>(static_cast<const double2*>(W), w_batch, wi, wj, Kin, L.Kh, Nout,
-                                                   L.Npad, db, static_cast<int>(L.ld), ew);
+                                                   L.Npad, db, static_cast<int>(L.ld), eb, ew);
   QGB_LAUNCH_CHECK("k_oz_slice_mat");
-  for (int pan = 0; pan < L.panels; ++pan) {
+  // The last panel first: its part of X is the one k_oz_band_exp left in L2.
+  for (int pan = L.panels - 1; pan >= 0; --pan) {
     const int g0 = pan * L.rows;
     const int rows = std::min(L.rows, G - g0);
     k_oz_slice_cols<<<dim3((rows + 31) / 32, nk), 256, 0, st>>>(static_cast<const double2*>(X), x_batch, ldx, Kin, L.Kh,
-                                                               g0, G, rows, da, static_cast<int>(L.ld), eg,
-                                                               pan == 0 ? err : nullptr);
+                                                               g0, G, rows, da, static_cast<int>(L.ld), eb, eg,
+                                                               pan == L.panels - 1 ? err : nullptr);
     QGB_LAUNCH_CHECK("k_oz_slice_cols");
     GemmArgs g{};
     g.chunks = L.chunks;
