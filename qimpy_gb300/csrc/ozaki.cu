@@ -84,9 +84,9 @@ struct GemmArgs {
   int a_rows, b_rows;      // complex rows; real row r belongs to r % a_rows / b_rows (EPI_PARTIAL)
   int M, N;                // real rows of A and B
   int* err;
-  // EPI_PARTIAL: FP64 [split][batch][M][N]
+  // EPI_PARTIAL: FP64 [split][batch][M][N], this panel's from split0 on; add: to the earlier panels' sums
   double* partial;
-  int split0, nbatch;
+  int split0, add, nbatch;
   // EPI_ROTATE: rows g0 + row < G; band j of column c (see k_oz_slice_mat)
   double2* out;
   long long out_batch;
@@ -381,8 +381,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             const int row = t.m_tile * BM + (warp & 3) * 32 + r;
             if (row < args.M && col < args.N) {
               const longlong2 v = sums[cc * SUMS_LD + r];
-              out[static_cast<long long>(row) * args.N + col] =
-                  ok ? to_double(v.x, v.y, ec + ea[row % args.a_rows]) : nan;
+              double* o = out + static_cast<long long>(row) * args.N + col;
+              const double d = ok ? to_double(v.x, v.y, ec + ea[row % args.a_rows]) : nan;
+              *o = args.add ? *o + d : d;
             }
           }
         } else {
@@ -701,14 +702,14 @@ __global__ void __launch_bounds__(128) k_oz_slice_mat(const double2* __restrict_
 // P[M + i][j] of the stacked real products (fold: the real part alone).  They
 // are added as 64-bit integers in units of 2^-54 of the largest, which costs
 // the FP64 pipe nothing and rounds once (two terms below 2^55 of each of at most
-// kMaxSplits splits stay below 2^63).  Rows marked non-finite are computed here
-// by multiply-adds.
+// kMaxSplits sets stay below 2^63).  Rows marked non-finite in any split of any
+// panel (`exps` of them) are computed here by multiply-adds.
 constexpr int kRed = 8;  // threads per output, over the splits
 template <int FOLD>
 __global__ void __launch_bounds__(256)
-    k_oz_reduce(const double* __restrict__ partial, int splits, int nbatch, int M, int N, double2* __restrict__ out,
-                long long out_batch, int oi, int oj, const int* __restrict__ ea, const int* __restrict__ eb,
-                int panel_splits, const double2* __restrict__ A, const double2* __restrict__ B, long long a_batch,
+    k_oz_reduce(const double* __restrict__ partial, int sets, int panel_splits, int nbatch, int M, int N,
+                double2* __restrict__ out, long long out_batch, int oi, int oj, const int* __restrict__ ea, const int* __restrict__ eb,
+                int exps, const double2* __restrict__ A, const double2* __restrict__ B, long long a_batch,
                 long long b_batch, int lda, int ldb, int K, const double* __restrict__ weight) {
   const long long per = static_cast<long long>(M) * N;
   const int R = FOLD ? 1 : 2;
@@ -722,11 +723,13 @@ __global__ void __launch_bounds__(256)
     const double* P1 = P0 + static_cast<long long>(M) * R * N;  // the Im rows (not folded)
     int er = 1, ei = 1;
     bool bad = false;
-    for (int s = sub; s < splits; s += kRed) {
+    for (int s = sub; s < exps; s += kRed) {
       // The exponents are kept per panel, [batch][panel_splits][rows] each.
       const int pan = s / panel_splits, ps = s - pan * panel_splits;
       const long long es = (static_cast<long long>(pan) * nbatch + k) * panel_splits + ps;
       bad |= ea[es * M + i] == kNonFinite || eb[es * N + j] == kNonFinite;
+    }
+    for (int s = sub; s < sets; s += kRed) {
       er = max(er, exp_field(P0[s * per_split]));
       if (!FOLD) {
         er = max(er, exp_field(P1[s * per_split + N]));
@@ -738,7 +741,7 @@ __global__ void __launch_bounds__(256)
     bad = __any_sync(lanes, bad);
     long long sr = 0, si = 0;
     if (!bad && max(er, ei) != kNonFinite) {
-      for (int s = sub; s < splits; s += kRed) {
+      for (int s = sub; s < sets; s += kRed) {
         sr += fixed_point(P0[s * per_split], er);
         if (!FOLD) {
           sr += fixed_point(P1[s * per_split + N], er);
@@ -769,7 +772,7 @@ __global__ void __launch_bounds__(256)
         im = fma(-u.y, v.x, im);
       }
     } else if (max(er, ei) == kNonFinite) {  // a product overflowed, or a pipeline wait ran out
-      for (int s = 0; s < splits; ++s) {
+      for (int s = 0; s < sets; ++s) {
         re += FOLD ? P0[s * per_split] : P0[s * per_split] + P1[s * per_split + N];
         if (!FOLD) im += P0[s * per_split + N] - P1[s * per_split];
       }
@@ -786,9 +789,17 @@ __global__ void __launch_bounds__(256)
 // Host: plans and launches
 // ---------------------------------------------------------------------------
 
-// Digits of one panel stay below this, so that a workspace is bounded for any
-// basis and most of a panel's digits are read back from L2.
+// An operand is sliced in panels, of K for an overlap and of g for a rotation,
+// whose digits stay below kPanelBytes (an overlap's panel takes at least
+// kPanelChunks chunks of K: 28 B per value of 512 columns, below its operands from
+// K = 900 on).  So a workspace is bounded, and most of a panel's digits are read
+// back from L2.  (W of a rotation is sliced whole, 3.5 times its size.)  Every panel
+// of an overlap has partial sums of its own while all of them stay below
+// kPanelBytes too; otherwise the panels add into one set, of one wave of CTAs or of
+// twice the output's size, which costs a panel some 5 us of reads (352 x 176 over
+// 37073, 5 panels: 810 us in 45 sets, 837 us in 9).
 constexpr long long kPanelBytes = 128ll << 20;
+constexpr int kPanelChunks = 4;
 constexpr int kMaxSplits = 127;  // partial sums of an overlap, see k_oz_reduce
 
 // bf16 digits [batch][7][rows][ld], box 64 x box_rows of one digit with 128-byte
@@ -826,8 +837,8 @@ static int launch_gemm(const void* a, long long a_rows, const void* b, long long
 
 struct OzGram {
   long long a_rows, b_rows;     // real rows
-  int fold, tiles, Lg, chunks;  // g per split, K chunks per split
-  int panel_splits, panels;
+  int fold, Lg, chunks;         // g per split, K chunks per split
+  int panel_splits, panels, sets;  // sets of partial sums: one a split of a panel, or of all panels
   long long ld, a_elems, b_elems;
   size_t digits_bytes, e_bytes, partial_bytes, total;
 };
@@ -838,27 +849,29 @@ static OzGram gram_layout(int nk, int M, int N, int K, bool real_out) {
   L.a_rows = real_out ? M : 2ll * M;
   L.b_rows = real_out ? N : 2ll * N;
   const long long mt = (L.a_rows + BM - 1) / BM, nt = (L.b_rows + BN - 1) / BN;
-  L.tiles = static_cast<int>(mt * nt * nk);
   const int gpc = L.fold ? CHUNK / 2 : CHUNK;  // g per K chunk
   const int nchunk = (K + gpc - 1) / gpc;
   const long long per_chunk = nk * (L.a_rows + L.b_rows) * CHUNK * S * 2;
-  const int cap = static_cast<int>(std::max<long long>((nchunk + kMaxSplits - 1) / kMaxSplits,
-                                                       std::min<long long>(nchunk, kPanelBytes / per_chunk)));
+  const int cap = static_cast<int>(std::min<long long>(nchunk, std::max<long long>(kPanelChunks, kPanelBytes / per_chunk)));
   L.panels = (nchunk + cap - 1) / cap;
   const int cpp = (nchunk + L.panels - 1) / L.panels;
   // One wave of CTAs over the SMs per panel (one CTA fills an SM).
-  const int want = std::max(1, std::min({cpp, kSms / L.tiles, kMaxSplits / L.panels}));
+  const int want = static_cast<int>(std::max(1ll, std::min({static_cast<long long>(cpp), kSms / (mt * nt * nk),
+                                                            static_cast<long long>(kMaxSplits)})));
   L.chunks = (cpp + want - 1) / want;
   L.panel_splits = (cpp + L.chunks - 1) / L.chunks;
   L.Lg = L.chunks * gpc;
-  L.panels = (K + L.Lg * L.panel_splits - 1) / (L.Lg * L.panel_splits);
+  L.panels = static_cast<int>((K + static_cast<long long>(L.Lg) * L.panel_splits - 1) /
+                              (static_cast<long long>(L.Lg) * L.panel_splits));
   L.ld = static_cast<long long>(L.panel_splits) * L.chunks * CHUNK;
   L.a_elems = round_up(nk * S * L.a_rows * L.ld, 128);
   L.b_elems = round_up(nk * S * L.b_rows * L.ld, 128);
   L.digits_bytes = static_cast<size_t>(L.a_elems + L.b_elems) * 2;
   const long long splits = static_cast<long long>(L.panels) * L.panel_splits;
   L.e_bytes = static_cast<size_t>(round_up(splits * nk * (M + N) * 4, 256));
-  L.partial_bytes = static_cast<size_t>(round_up(splits * nk * L.a_rows * L.b_rows * 8, 256));
+  const long long set_bytes = nk * L.a_rows * L.b_rows * 8;
+  L.sets = static_cast<int>(splits <= kMaxSplits && splits * set_bytes <= kPanelBytes ? splits : L.panel_splits);
+  L.partial_bytes = static_cast<size_t>(round_up(L.sets * set_bytes, 256));
   L.total = L.digits_bytes + L.e_bytes + L.partial_bytes + 256 + 256;
   return L;
 }
@@ -950,15 +963,17 @@ int oz_gram(const void* A, long long a_batch, int lda, const void* B, long long 
     g.N = static_cast<int>(L.b_rows);
     g.err = err;
     g.partial = partial;
-    g.split0 = pan * L.panel_splits;
+    const bool own = L.sets > L.panel_splits;  // (one panel: either)
+    g.split0 = own ? pan * L.panel_splits : 0;
+    g.add = !own && pan > 0 ? 1 : 0;
     g.nbatch = nk;
     if (int rc = launch_gemm<EPI_PARTIAL>(da, L.a_rows, db, L.b_rows, nk, L.ld, g, st)) return rc;
   }
   const long long total = static_cast<long long>(nk) * M * N;
   const unsigned blocks = static_cast<unsigned>(std::min<long long>((total * kRed + 255) / 256, 8 * kSms));
   auto* reduce = L.fold ? k_oz_reduce<1> : k_oz_reduce<0>;
-  reduce<<<blocks, 256, 0, st>>>(partial, static_cast<int>(splits), nk, M, N, static_cast<double2*>(out), out_batch, oi,
-                                 oj, ea, eb, L.panel_splits, static_cast<const double2*>(A),
+  reduce<<<blocks, 256, 0, st>>>(partial, L.sets, L.panel_splits, nk, M, N, static_cast<double2*>(out), out_batch, oi,
+                                 oj, ea, eb, static_cast<int>(splits), static_cast<const double2*>(A),
                                  static_cast<const double2*>(B), a_batch, b_batch, lda, ldb, K, weight);
   QGB_LAUNCH_CHECK("k_oz_reduce");
   return QGB_OK;
