@@ -180,7 +180,9 @@ __global__ void k_gram_reduce(const cplx_t<T>* __restrict__ partial, int splits,
 // sums are folded across the lanes (each step halves the values a lane keeps,
 // so TI TJ complex sums cost about as many additions) and then the 8 warps.
 // The 64 x 64 tiles above would multiply padding and leave most SMs idle (k = 8
-// times 8 x 18 outputs over 1150 g: 517 us against 14 us here).
+// times 8 x 18 outputs over 1150 g: 517 us against 14 us here).  A few outputs
+// over a long basis are split over g as well (launch_gram_small): 4 x 3 over
+// 37073 is 4 tiles, 148 us on as many SMs, 11 us in 38 parts.
 template <typename T, typename OutT, int TI, int TJ>
 __global__ void __launch_bounds__(256) k_gram_small(const GramArgs a) {
   using C2 = cplx_t<T>;
@@ -188,7 +190,8 @@ __global__ void __launch_bounds__(256) k_gram_small(const GramArgs a) {
   constexpr int V = 2 * TI * TJ;
   __shared__ Acc red[8][V];
   const int nj = (a.N + TJ - 1) / TJ;
-  const int i0 = (blockIdx.x / nj) * TI, j0 = (blockIdx.x % nj) * TJ, k = blockIdx.y;
+  const int i0 = (blockIdx.x / nj) * TI, j0 = (blockIdx.x % nj) * TJ, k = blockIdx.y, split = blockIdx.z;
+  const int g_end = min(a.K, (split + 1) * a.g_per_split);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const C2* A = static_cast<const C2*>(a.A) + k * a.a_batch;
   const C2* B = static_cast<const C2*>(a.B) + k * a.b_batch;
@@ -197,7 +200,7 @@ __global__ void __launch_bounds__(256) k_gram_small(const GramArgs a) {
   for (int p = 0; p < TI; ++p)
 #pragma unroll
     for (int q = 0; q < TJ; ++q) acc[p][q] = mk<T>(T(0), T(0));
-  for (int g = threadIdx.x; g < a.K; g += 256) {
+  for (int g = split * a.g_per_split + threadIdx.x; g < g_end; g += 256) {
     C2 av[TI], bv[TJ];
 #pragma unroll
     for (int p = 0; p < TI; ++p) av[p] = A[static_cast<long long>(min(i0 + p, a.M - 1)) * a.lda + g];
@@ -250,11 +253,39 @@ __global__ void __launch_bounds__(256) k_gram_small(const GramArgs a) {
       re += red[w][2 * threadIdx.x];
       im += red[w][2 * threadIdx.x + 1];
     }
-    if (i < a.M && j < a.N)
+    if (i >= a.M || j >= a.N) return;
+    if (a.splits > 1)
+      static_cast<cplx_t<Acc>*>(a.partial)[((static_cast<long long>(split) * gridDim.y + k) * a.M + i) * a.N + j] =
+          mk<Acc>(re, im);
+    else
       static_cast<cplx_t<OutT>*>(a.out)[k * a.out_batch + static_cast<long long>(i) * a.oi +
                                         static_cast<long long>(j) * a.oj] =
           mk<OutT>(static_cast<OutT>(re), a.real_out ? OutT(0) : static_cast<OutT>(im));
   }
+}
+
+// Sum of its partials: a warp an output, lane l those of splits l, l + 32, ...
+template <typename T, typename OutT>
+__global__ void __launch_bounds__(256) k_gram_small_reduce(const GramArgs a, int nk) {
+  using Acc = typename std::conditional<sizeof(T) >= sizeof(OutT), T, OutT>::type;
+  const long long per_k = static_cast<long long>(a.M) * a.N, e = blockIdx.x * 8ll + (threadIdx.x >> 5);
+  if (e >= per_k * nk) return;
+  const int lane = threadIdx.x & 31;
+  Acc re = 0, im = 0;
+  for (int s = lane; s < a.splits; s += 32) {
+    const cplx_t<Acc> v = static_cast<const cplx_t<Acc>*>(a.partial)[s * per_k * nk + e];
+    re += v.x;
+    im += v.y;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    re += __shfl_xor_sync(0xffffffffu, re, o);
+    im += __shfl_xor_sync(0xffffffffu, im, o);
+  }
+  const long long k = e / per_k, r = e - k * per_k, i = r / a.N, j = r - i * a.N;
+  if (lane == 0)
+    static_cast<cplx_t<OutT>*>(a.out)[k * a.out_batch + i * a.oi + j * a.oj] =
+        mk<OutT>(static_cast<OutT>(re), a.real_out ? OutT(0) : static_cast<OutT>(im));
 }
 
 struct GramPlan {
@@ -477,9 +508,9 @@ static void launch_gram(int shape, dim3 grid, const GramArgs& g, cudaStream_t st
 }
 
 // Products small enough that the FP64 pipe of all SMs takes about as long as
-// the launches of the sliced form.
-static bool small_product(int nk, int M, int N, int K) {
-  return static_cast<double>(nk) * M * N * K < 3e6 && nk <= 65535;
+// the launches of the sliced form (ozaki.cu has both sides).
+static bool small_product(int nk, int M, int N, int K, double limit = kSmallOverlap) {
+  return static_cast<double>(nk) * M * N * K < limit && nk <= 65535;
 }
 
 // Work of the SM that gets the most of `ctas` equal CTAs.  `work` counts an
@@ -491,21 +522,54 @@ static long long most_loaded(long long ctas, int work) { return (ctas + kSms - 1
 // The tile that loads the fullest SM least, the larger one on a tie: 8 x 18
 // outputs of 8 k are 160 tiles of 2 x 4, two on 8 of the SMs, or 288 of 2 x 2,
 // also two but half the size (1150 g, FP64: 23.7 -> 13.6 us).
+// g is split where the tiles leave SMs idle, into as many parts as give no SM two
+// of them, if that saves more than the second launch costs (9000 clocks): 256 g
+// take a tile 512 clocks per output in FP64, 250 in all in FP32.  One part and
+// split, us: 4 x 3 over 37073 FP64 148 and 11 (FP32 23 and 7), 16 x 16 over 10000 44
+// and 27 (FP32, not split: 9.0 and 9.0), 18 x 18 over 8000 FP32, not split: 7.8 and 11.
+struct GramSmall {
+  int ti, tj, splits, g_per_split;
+};
+static GramSmall pick_gram_small(bool f64, int nk, int M, int N, int K, int max_splits) {
+  GramSmall best{4, 4, 1, K};
+  long long least = -1, ctas = 0;
+  for (const GramSmall& c : {GramSmall{4, 4, 1, K}, GramSmall{2, 4, 1, K}, GramSmall{2, 2, 1, K}}) {
+    const long long n = static_cast<long long>((M + c.ti - 1) / c.ti) * ((N + c.tj - 1) / c.tj) * nk;
+    const long long cost = most_loaded(n, f64 ? c.ti * c.tj : c.ti * c.tj + 2 * (c.ti + c.tj));
+    if (least < 0 || cost < least) {
+      least = cost;
+      best = c;
+      ctas = n;
+    }
+  }
+  const long long iterations = (K + 255) / 256;
+  const long long s = std::min({static_cast<long long>(max_splits), iterations, kSms / ctas});
+  if (s > 1 && (iterations - iterations / s) * (f64 ? 512 * best.ti * best.tj : 250) > 9000)
+    best.g_per_split = static_cast<int>((iterations + s - 1) / s) * 256;
+  best.splits = (K + best.g_per_split - 1) / best.g_per_split;
+  return best;
+}
+
 template <typename T, typename OutT>
-static void launch_gram_small(const GramArgs& g, int nk, cudaStream_t st) {
-  const auto ctas = [&](int ti, int tj) {
-    return static_cast<unsigned>((g.M + ti - 1) / ti) * static_cast<unsigned>((g.N + tj - 1) / tj);
-  };
-  const auto cost = [&](int ti, int tj) {
-    return most_loaded(static_cast<long long>(ctas(ti, tj)) * nk,
-                       sizeof(T) == 8 ? ti * tj : ti * tj + 2 * (ti + tj));
-  };
-  if (cost(4, 4) <= std::min(cost(2, 4), cost(2, 2)))
-    k_gram_small<T, OutT, 4, 4><<<dim3(ctas(4, 4), nk), 256, 0, st>>>(g);
-  else if (cost(2, 4) <= cost(2, 2))
-    k_gram_small<T, OutT, 2, 4><<<dim3(ctas(2, 4), nk), 256, 0, st>>>(g);
+static int launch_gram_small(GramArgs g, int nk, int max_splits, cudaStream_t st) {
+  const GramSmall p = pick_gram_small(sizeof(T) == 8, nk, g.M, g.N, g.K, max_splits);
+  g.splits = p.splits;
+  g.g_per_split = p.g_per_split;
+  const dim3 grid(static_cast<unsigned>((g.M + p.ti - 1) / p.ti) * static_cast<unsigned>((g.N + p.tj - 1) / p.tj), nk,
+                  p.splits);
+  if (p.ti == 4)
+    k_gram_small<T, OutT, 4, 4><<<grid, 256, 0, st>>>(g);
+  else if (p.tj == 4)
+    k_gram_small<T, OutT, 2, 4><<<grid, 256, 0, st>>>(g);
   else
-    k_gram_small<T, OutT, 2, 2><<<dim3(ctas(2, 2), nk), 256, 0, st>>>(g);
+    k_gram_small<T, OutT, 2, 2><<<grid, 256, 0, st>>>(g);
+  QGB_LAUNCH_CHECK("k_gram_small");
+  if (p.splits > 1) {
+    const long long outputs = static_cast<long long>(nk) * g.M * g.N;
+    k_gram_small_reduce<T, OutT><<<static_cast<unsigned>((outputs + 7) / 8), 256, 0, st>>>(g, nk);
+    QGB_LAUNCH_CHECK("k_gram_small_reduce");
+  }
+  return QGB_OK;
 }
 
 // Columns a thread and threads a CTA of k_rotate_small, by the same rule: 4, 2 or
@@ -558,16 +622,14 @@ int gram(int dtype, int out_dtype, const void* A, long long a_batch, int lda, co
       ws_bytes >= oz_gram_workspace_bytes(nk, M, N, K, real_out))
     return oz_gram(A, a_batch, lda, B, b_batch, ldb, nk, M, N, K, out, out_batch, oi, oj, ws, st, weight, real_out);
   if (small_product(nk, M, N, K)) {
-    const GramArgs g{A, B, a_batch, b_batch, lda, ldb, M, N, K, 1, K, nullptr, out, out_batch, oi, oj, weight,
+    const GramArgs g{A, B, a_batch, b_batch, lda, ldb, M, N, K, 1, K, ws, out, out_batch, oi, oj, weight,
                      real_out ? 1 : 0};
-    if (dtype == QGB_F64)
-      launch_gram_small<double, double>(g, nk, st);
-    else if (out_dtype == QGB_F64)
-      launch_gram_small<float, double>(g, nk, st);
-    else
-      launch_gram_small<float, float>(g, nk, st);
-    QGB_LAUNCH_CHECK("k_gram_small");
-    return QGB_OK;
+    // Its partial sums have the result's precision; the workspace holds p.splits of the operands'.
+    const size_t acc = elem_bytes(out_dtype);
+    const int room = reinterpret_cast<uintptr_t>(ws) % acc ? 1 : static_cast<int>(p.splits * elem_bytes(dtype) / acc);
+    if (dtype == QGB_F64) return launch_gram_small<double, double>(g, nk, std::max(1, room), st);
+    if (out_dtype == QGB_F64) return launch_gram_small<float, double>(g, nk, std::max(1, room), st);
+    return launch_gram_small<float, float>(g, nk, std::max(1, room), st);
   }
   GramArgs g{A, B, a_batch, b_batch, lda, ldb, M, N, K, p.splits, p.g_per_split, ws, out, out_batch, oi, oj,
              weight, real_out ? 1 : 0};
@@ -609,7 +671,7 @@ int rotate(int dtype, const void* X, long long x_batch, int ldx, const void* W, 
       ws_bytes >= oz_rotate_workspace_bytes(nk, Kin, Nout, G))
     return oz_rotate(X, x_batch, ldx, W, w_batch, wi, wj, nk, Kin, Nout, G, out, out_batch, ldo, accumulate, ws, st);
   RotArgs r{X, W, out, x_batch, w_batch, out_batch, ldx, ldo, wi, wj, Kin, Nout, G, accumulate ? 1 : 0};
-  if (small_product(nk, Kin, Nout, G) && (Nout + 3) / 4 <= 65535 && (dtype == QGB_F64 || dtype == QGB_F32)) {
+  if (small_product(nk, Kin, Nout, G, kSmallRotation) && (Nout + 3) / 4 <= 65535 && (dtype == QGB_F64 || dtype == QGB_F32)) {
     const RotSmall c = pick_rotate_small(dtype, nk, Nout, G);
     if (dtype == QGB_F64)
       launch_rotate_small<double, false>(r, nk, nullptr, 0, c, st);

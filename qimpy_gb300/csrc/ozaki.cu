@@ -906,18 +906,18 @@ static OzRot rot_layout(int nk, int Kin, int Nout, int G) {
 
 using namespace oz;
 
-// Where the sliced product is the faster form.  Its launches and fills take
-// 30-40 us whatever the size, the multiply-adds' time grows with the product:
-//   overlap   18 x 18 x 8000 (2.6 M multiply-adds)  sliced 45 us, multiply-adds 37 us
+// Where the sliced product is the faster form (kSmallOverlap, kSmallRotation).  Its
+// launches and fills take 30-40 us whatever the size, the multiply-adds' time grows
+// with the product:
+//   overlap   18 x 18 x 8000 (2.6 M multiply-adds)  sliced 45 us, multiply-adds 35 us
 //             8 k of 36 x 18 x 1150 (6 M)           43 us against 66 us
-//   rotation  the same two sizes                    33 against 27 us, 35 against 51 us
-static bool oz_worth(double macs) { return macs >= 3e6; }
-
+//   rotation  60 x 60 x 1000 (3.6 M)                33 us against 30 us
+//             64 x 64 x 1000 (4.1 M)                33 us against 36 us
 bool oz_gram_use(int nk, int M, int N, int K) {
-  return oz_worth(static_cast<double>(nk) * M * N * K) && nk <= 4096 && M <= 65535 && N <= 65535;
+  return static_cast<double>(nk) * M * N * K >= kSmallOverlap && nk <= 4096 && M <= 65535 && N <= 65535;
 }
 bool oz_rotate_use(int nk, int Kin, int Nout, int G) {
-  return oz_worth(static_cast<double>(nk) * Kin * Nout * G) && nk <= 4096 && Nout <= 65535 &&
+  return static_cast<double>(nk) * Kin * Nout * G >= kSmallRotation && nk <= 4096 && Nout <= 65535 &&
          G <= 65535 * kExpRange;
 }
 
