@@ -28,7 +28,7 @@ int rotate(int dtype, const void* X, long long x_batch, int ldx, const void* W, 
 
 // FP64 products by integer slices on the tensor cores (ozaki.cu), from these many
 // multiply-adds on; smaller ones take the small kernels.
-constexpr double kSmallOverlap = 3e6, kSmallRotation = 3e6;
+constexpr double kSmallOverlap = 3e6, kSmallRotation = 4e6;
 bool oz_gram_use(int nk, int M, int N, int K);
 size_t oz_gram_workspace_bytes(int nk, int M, int N, int K, bool real_out);
 int oz_gram(const void* A, long long a_batch, int lda, const void* B, long long b_batch, int ldb, int nk, int M, int N,
