@@ -73,12 +73,15 @@ int violation_local_f32(unsigned long long*);
 int violation_local_f64(unsigned long long*);
 int violation_batched_f32(unsigned long long*);
 int violation_batched_f64(unsigned long long*);
+int violation_density_f32(unsigned long long*);
+int violation_density_f64(unsigned long long*);
 // Debug builds: copy out and clear the first recorded range violation
 // (site, index, limit, packed block index); site 0 = none.
 int debug_violation(unsigned long long* out4) {
   QGB_CUDA_CHECK(cudaDeviceSynchronize());
   for (int i = 0; i < 4; ++i) out4[i] = 0;
-  for (auto* unit : {violation_local_f32, violation_local_f64, violation_batched_f32, violation_batched_f64})
+  for (auto* unit : {violation_local_f32, violation_local_f64, violation_batched_f32, violation_batched_f64,
+                     violation_density_f32, violation_density_f64})
     if (int rc = unit(out4)) return rc;
   return QGB_OK;
 }
