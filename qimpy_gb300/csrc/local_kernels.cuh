@@ -255,7 +255,7 @@ __device__ __forceinline__ void body_ifft_yz(const qgb_sphere& s, const LocalPar
 #pragma unroll
     for (int u = 0; u < kPoints; ++u) {
       const int g = gb + u * blockDim.x;
-      v[u] = g < g1 ? yz[g] : 0;
+      v[u] = g < g1 && QGB_OK_IDX(g, s.n[k], 1) ? yz[g] : 0;
     }
 #pragma unroll
     for (int u = 0; u < kPoints; ++u) {
@@ -454,7 +454,7 @@ __device__ __forceinline__ void x_tables(const qgb_sphere& s, const int k, const
   const int* i0 = s.slab_i0 + k * s.max_slabs;
   for (int sl = threadIdx.x; sl < s.n_slabs[k]; sl += blockDim.x) {
     const int x = i0[sl];
-    if (QGB_OK_IDX(x, N0, 63)) xs[x] = sl * s.N[1] * s.N[2];
+    if (QGB_OK_IDX(x, N0, 63) && QGB_OK_IDX(sl, s.max_slabs, 6)) xs[x] = sl * s.N[1] * s.N[2];
   }
   __syncthreads();
 }
@@ -478,6 +478,7 @@ __device__ __forceinline__ void body_xpass(const qgb_sphere& s, const LocalParam
   C2* sm = smem_c<T>();
   int* xs = reinterpret_cast<int*>(sm + Wx + N0);
   const size_t plane = static_cast<size_t>(N1) * N2;
+  if (!QGB_OK_IDX(plane_index(s, k, b, lp.nb, 0), (long long)s.nk * lp.nb * s.max_slabs, 5)) return;
   C2* base = planes + plane_index(s, k, b, lp.nb, 0) * plane + c0;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   if (L2 > 1) {
@@ -492,7 +493,9 @@ __device__ __forceinline__ void body_xpass(const qgb_sphere& s, const LocalParam
   // V[p0][c0 + c] with p0 = a * L1 + j: j-stride N1 * N2.
   const T* V = static_cast<const T*>(s.V) + c0;
   x_items<W32>(nz, L2, [&](int a, int c) {
-    if (!QGB_OK_IDX(c + (a * L1 + L1 - 1) * ld, lim, 7) || !QGB_OK_IDX((L1 - 1) * L2 + a, N0, 9)) return;
+    if (!QGB_OK_IDX(c + (a * L1 + L1 - 1) * ld, lim, 7) || !QGB_OK_IDX((L1 - 1) * L2 + a, N0, 9) ||
+        !QGB_OK_IDX(static_cast<long long>(a * L1 + L1 - 1) * plane + c0 + (W32 ? min(c, nz - 1) : c), N0 * plane, 8))
+      return;
     xmid_dispatch<T>(L1, sm, c + a * L1 * ld, ld, V + static_cast<unsigned>(a * L1 * N1 * N2 + (W32 ? min(c, nz - 1) : c)),
                      N1 * N2, Wx, L2, a);
   });
@@ -597,12 +600,13 @@ __device__ __forceinline__ void xpair_last_R(float2* __restrict__ base, const in
 }
 
 template <int R>
-__device__ __forceinline__ void xpair_mid_R(const float* __restrict__ V, const PairLane l, unsigned plane, int L2,
-                                            int Wx, int lim) {
+__device__ __forceinline__ void xpair_mid_R(const float* __restrict__ V, const PairLane l, unsigned plane, int v_lim,
+                                            int L2, int Wx, int lim) {
   cpair_t* sm = smem_pairs();
   const int v0 = l.in0 ? l.c : 0, v1 = l.in1 ? l.c + 32 : v0;  // lanes beyond the tile read V of its first columns
   x_items<true>(0, L2, [&](int a, int c) {
-    if (!QGB_OK_IDX(c + (a * R + R - 1) * 32, lim, 7)) return;
+    if (!QGB_OK_IDX(c + (a * R + R - 1) * 32, lim, 7) || !QGB_OK_IDX((a * R + R - 1) * plane + max(v0, v1), v_lim, 8))
+      return;
     cpair_t* p = sm + a * R * 32 + c;
     const float* Va = V + static_cast<unsigned>(a * R) * plane;
     PairBlock<R> x;
@@ -640,13 +644,13 @@ __device__ __forceinline__ void xpair_mid_R(const float* __restrict__ V, const P
 // STEP 0: first inverse pass (radix L2), 1: middle step (L1), 2: last forward (L2).
 template <int STEP>
 __device__ __forceinline__ void xpair_step(int R, float2* base, const float* V, const int* xs, const PairLane l,
-                                           unsigned plane, int L1, int L2, int Wx, int lim) {
+                                           unsigned plane, int v_lim, int L1, int L2, int Wx, int lim) {
 #define QGB_XP(RR)                                             \
   case RR:                                                     \
     if constexpr (STEP == 0)                                   \
       xpair_first_R<RR>(base, xs, l, L1, Wx, lim);             \
     else if constexpr (STEP == 1)                              \
-      xpair_mid_R<RR>(V, l, plane, L2, Wx, lim);               \
+      xpair_mid_R<RR>(V, l, plane, v_lim, L2, Wx, lim);        \
     else                                                       \
       xpair_last_R<RR>(base, xs, l, L1, lim);                  \
     break;
@@ -673,7 +677,7 @@ __device__ __forceinline__ void x_tables_pair(const qgb_sphere& s, const int k) 
   const int* i0 = s.slab_i0 + k * s.max_slabs;
   for (int sl = threadIdx.x; sl < s.n_slabs[k]; sl += blockDim.x) {
     const int x = i0[sl];
-    if (QGB_OK_IDX(x, N0, 63)) xs[x] = sl * s.N[1] * s.N[2];
+    if (QGB_OK_IDX(x, N0, 63) && QGB_OK_IDX(sl, s.max_slabs, 6)) xs[x] = sl * s.N[1] * s.N[2];
   }
   __syncthreads();
 }
@@ -685,12 +689,14 @@ __device__ __forceinline__ void body_xpass_pair(const qgb_sphere& s, const Local
   cpair_t* sm = smem_pairs();
   const int* xs = reinterpret_cast<const int*>(sm + lim + N0);
   const size_t plane = static_cast<size_t>(s.N[1]) * s.N[2];
+  if (!QGB_OK_IDX(plane_index(s, k, b, lp.nb, 0), (long long)s.nk * lp.nb * s.max_slabs, 5)) return;
   float2* base = planes + plane_index(s, k, b, lp.nb, 0) * plane + c0;
   const float* V = static_cast<const float*>(s.V) + c0;
+  const int v_lim = N0 * static_cast<int>(plane) - c0;  // V's elements from c0 on (range checks)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
   const PairLane l{lane, lane < nz, lane + 32 < nz};
   if (L2 > 1) {
-    xpair_step<0>(L2, base, V, xs, l, plane, L1, L2, lim, lim);
+    xpair_step<0>(L2, base, V, xs, l, plane, v_lim, L1, L2, lim, lim);
   } else {
     for (int x = warp; x < N0; x += nwarps) {
       const int o = xs[x];
@@ -698,10 +704,10 @@ __device__ __forceinline__ void body_xpass_pair(const qgb_sphere& s, const Local
     }
   }
   __syncthreads();
-  xpair_step<1>(L1, base, V, xs, l, plane, L1, L2, lim, lim);
+  xpair_step<1>(L1, base, V, xs, l, plane, v_lim, L1, L2, lim, lim);
   __syncthreads();
   if (L2 > 1) {
-    xpair_step<2>(L2, base, V, xs, l, plane, L1, L2, lim, lim);
+    xpair_step<2>(L2, base, V, xs, l, plane, v_lim, L1, L2, lim, lim);
   } else {
     for (int x = warp; x < N0; x += nwarps) {
       const int o = xs[x];
@@ -788,7 +794,7 @@ __device__ __forceinline__ void body_fft_yz_gather(const qgb_sphere& s, const Lo
 #pragma unroll
     for (int u = 0; u < kPoints; ++u) {
       const int g = gb + u * blockDim.x;
-      const bool in = g < g1;
+      const bool in = g < g1 && QGB_OK_IDX(g, s.n[k], 1);
       v[u] = in ? yz[g] : 0;
       c[u] = o[u] = mk<T>(T(0), T(0));
       e[u] = T(0);

@@ -20,3 +20,11 @@ def test_every_unit_with_checked_kernels_is_read():
     for u in checked:
         assert f"int violation_{u}(" in _text(u + ".cu"), u
         assert f"violation_{u}" in query, u
+
+
+def test_points_are_checked_before_their_tables_are_read():
+    """A sphere point's index is tested where it is first used, not after the loads."""
+    body = _text("local_kernels.cuh")
+    assert len(re.findall(r"g < g1 && QGB_OK_IDX\(g, s\.n\[k\], 1\)", body)) == 2
+    for site in (4, 5, 6, 8):  # planes of the y/z passes and of the x-pass, its slabs, V
+        assert re.search(rf"QGB_OK_IDX\([^;]*, {site}\)", body), site
