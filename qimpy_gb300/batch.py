@@ -183,10 +183,11 @@ class Instance:
         basis.ke = torch.from_numpy(self.layout.ke).to(self.sphere.device)
         basis.real = self.real_basis
         basis.weight = self.real_basis.weight if self.real_basis is not None else None
-        # Subspace products on the CUDA cores: the tensor-core ones take ~0.2 GB
-        # of bf16 operand workspace per call on the largest cells, and with many
-        # requests' worker threads each caching its own, served runs exhausted
-        # device memory (library handle creation then failed).
+        # Complex64 subspace products on the CUDA cores: the tensor-core ones take
+        # ~0.2 GB of bf16 operand workspace per call on the largest cells, and with
+        # many requests' worker threads each caching its own, served runs exhausted
+        # device memory (library handle creation then failed).  (The FP64 ones, at
+        # most some 128 MB of digits and sums, are in EigenServer.estimate_bytes.)
         basis.tc_subspace = False
         pad = torch.arange(basis.n_tot)[None, :] < torch.from_numpy(basis.n)[:, None]
         basis.mask = pad.to(self.sphere.device)

@@ -44,6 +44,19 @@ def workspace(nbytes: int, device) -> torch.Tensor:
     return torch.empty(max(int(nbytes), 1), dtype=torch.uint8, device=device)
 
 
+def fp64_product_bytes(nk: int, M: int, N: int, n: int) -> int:
+    """What an FP64 overlap of M with N vectors of length n, or a rotation of M to N
+    of them, takes as workspace at most (host arithmetic, for memory estimates;
+    the calls themselves ask the library)."""
+    if nk * M * N * n < 3e6:
+        return 32 * nk * M * N * min(304, n // 128 + 1)  # partial sums of the small kernels
+    panel = 128 << 20
+    digits = min(28 * nk * (M + N + 4) * (n + 128), max(panel, 28 * 512 * nk * (M + N + 4)))
+    sums = max(min(32 * nk * M * N * (n // 128 + 1), panel), 32 * nk * M * N)
+    matrix = 56 * nk * (M + 4) * (N + 32)
+    return digits + max(sums, matrix) + 4 * nk * (M + N + 64) * (n // 64 + 2) + 4 * nk * n + 4096
+
+
 def apply_ke(sphere: DeviceSphere, C: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
     nb = _check_wf(sphere, C)
     out = torch.empty_like(C) if out is None else out

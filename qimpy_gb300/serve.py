@@ -146,7 +146,9 @@ class EigenServer:
     # ------------------------------------------------------------------ admission
     def estimate_bytes(self, spec: InstanceSpec, n_bands: int) -> int:
         """HBM held by an active request: wavefunction-sized Davidson arrays, the
-        slab planes of one block, projectors (and their bf16 operands), V, tables."""
+        slab planes of one block, projectors (and their bf16 operands), V, tables,
+        and the workspace its FP64 products (subspace and projections; the
+        refinement's for a mixed request) leave cached on its stream."""
         N = spec.grid
         nk = len(spec.k)
         n_est = (2.0 * spec.ke_cutoff) ** 1.5 * spec.side ** 3 / (6 * math.pi ** 2) * 1.1
@@ -156,7 +158,8 @@ class EigenServer:
         planes = nk * nbt * (N // 2 + 2) * N * N * elem
         P = 4 * spec.n_atoms
         proj = nk * P * n_est * (elem + (8 if self.dtype == torch.complex64 else 0))
-        return int(wf + planes + proj + 4 * N ** 3 * 8)
+        products = max(ops.fp64_product_bytes(nk, rows, nbt, int(n_est)) for rows in (2 * nbt, P))
+        return int(wf + planes + proj + 4 * N ** 3 * 8 + products)
 
     def submit(self, req: EigenRequest) -> None:
         self.queue.append(req)

@@ -1,10 +1,13 @@
 """Workspaces of the FP64 band products stay in proportion to their operands and
 results, at any size (host arithmetic of the built library; no GPU)."""
 import os
+import types
 
+import numpy as np
 import pytest
+import torch
 
-from qimpy_gb300 import _lib
+from qimpy_gb300 import _lib, ops
 
 pytestmark = pytest.mark.skipif(not os.path.exists(_lib.LIB_PATH), reason="library not built")
 
@@ -43,3 +46,25 @@ def test_projection_and_back_projection():
         both = max(lib.qgb_dot_fast_workspace_bytes(_lib.QGB_F64, nk, P, nb, n),
                    lib.qgb_matmul_workspace_bytes(_lib.QGB_F64, nk, P, nb, n))
         assert both < 3 * PANEL
+
+
+@pytest.mark.parametrize("nk,M,N,K", SIZES + [(1, 1, 1, 1), (2, 12, 6, 300), (8, 36, 18, 1150), (1, 24, 12, 900),
+                                              (4, 400, 200, 20000), (1, 256, 32, 37073), (1, 16, 3, 100000)])
+def test_estimate_covers_what_the_calls_ask_for(nk, M, N, K):
+    lib = _lib.lib()
+    asked = max(lib.qgb_dot_fast_workspace_bytes(_lib.QGB_F64, nk, M, N, K),
+                lib.qgb_matmul_workspace_bytes(_lib.QGB_F64, nk, M, N, K))
+    assert asked <= ops.fp64_product_bytes(nk, M, N, K)
+
+
+def test_served_requests_count_their_products():
+    from qimpy_gb300 import batch as bt, serve as sv
+
+    spec = bt.make_batch_specs(count=1, seed=3)[0]
+    for dtype in (torch.complex64, torch.complex128):
+        fake = types.SimpleNamespace(dtype=dtype, bands_extra=lambda nb, n: nb // 10 + 1)
+        need = sv.EigenServer.estimate_bytes(fake, spec, 64)
+        n = int((2.0 * spec.ke_cutoff) ** 1.5 * spec.side**3 / (6 * np.pi**2) * 1.1)
+        nbt, elem = 71, 8 if dtype == torch.complex64 else 16
+        held = 12 * len(spec.k) * nbt * n * elem + len(spec.k) * nbt * (spec.grid // 2 + 2) * spec.grid**2 * elem
+        assert need >= held + _lib.lib().qgb_dot_fast_workspace_bytes(_lib.QGB_F64, len(spec.k), 2 * nbt, nbt, n)
