@@ -158,7 +158,8 @@ class EigenServer:
         planes = nk * nbt * (N // 2 + 2) * N * N * elem
         P = 4 * spec.n_atoms
         proj = nk * P * n_est * (elem + (8 if self.dtype == torch.complex64 else 0))
-        products = max(ops.fp64_product_bytes(nk, rows, nbt, int(n_est)) for rows in (2 * nbt, P))
+        nbp = min(nbt, int(n_est) // 2)  # more are rejected
+        products = max(ops.fp64_product_bytes(nk, rows, nbp, int(n_est)) for rows in (2 * nbp, P))
         return int(wf + planes + proj + 4 * N ** 3 * 8 + products)
 
     def submit(self, req: EigenRequest) -> None:
