@@ -222,8 +222,11 @@ int qgb_project(int dtype, const void* beta, const void* C, void* projT, int nk,
  * (qimpy/dft/electrons/_wavefunction_dot.py:18-107).  Workspace of
  * qgb_dot_workspace_bytes (split-K partials, fixed summation order, so repeated
  * calls give equal bits).  With qgb_dot_fast_workspace_bytes (>= that) the larger
- * FP64 products run on the tensor cores as integer slices, to FP64 accuracy;
- * this holds for qgb_project (nx = P, ny = nb) and qgb_dot_real (nk = 1) too.
+ * FP64 products run on the tensor cores, on operands of 55 bits relative to the
+ * largest entry of each row (within a range of g): the error is that of FP64
+ * relative to max|X_i| max|Y_j|, where the smaller workspace's multiply-adds keep to
+ * sum_g |X_i| |Y_j|.  This holds for qgb_project (nx = P, ny = nb) and qgb_dot_real
+ * (nk = 1) too.
  */
 size_t qgb_dot_workspace_bytes(int dtype, int nk, int nx, int ny, int n_tot);
 size_t qgb_dot_fast_workspace_bytes(int dtype, int nk, int nx, int ny, int n_tot);
@@ -268,9 +271,11 @@ int qgb_dot_real(int dtype, const void* X, int nx, const void* Y, int ny, int n_
  * Wavefunction.matmul / @ (qimpy/dft/electrons/_wavefunction_dot.py:137-191).
  *
  * qgb_matmul_ws is the same with a workspace of qgb_matmul_workspace_bytes (0:
- * none needed), with which the larger FP64 rotations run on the tensor cores
- * (integer slices, FP64 accuracy); a smaller or NULL workspace, and qgb_matmul,
- * run on the FP64 pipe.
+ * none needed), with which the larger FP64 rotations run on the tensor cores, on
+ * operands of 55 bits relative to each band's largest entry: the error is that of
+ * FP64 relative to max_g |M_ij C_i(g)|, whatever the norms of the bands.  A smaller
+ * or NULL workspace, and qgb_matmul, run on the FP64 pipe (relative to
+ * sum_i |M_ij| |C_i(g)|).
  */
 int qgb_matmul(int dtype, const void* C, int n_in, int nk, int n_tot, const void* M, int n_out, void* out,
                unsigned flags, void* stream);

@@ -1,4 +1,4 @@
-// FP64 band-space products on the tensor cores, to full FP64 accuracy.
+// FP64 band-space products on the tensor cores, with 55-bit operands (see Accuracy).
 //
 // GB300's FP64 pipe runs 2 multiply-adds a cycle on each SM (1.2 TFLOP/s per
 // GPU), so the FP64 overlaps, projections and rotations were bound by it at
@@ -15,18 +15,34 @@
 //   below 2^24: 128 terms of at most 7 pairs, 128 * 7 * 2^14 < 2^24;
 //   after every 128 terms the 8 accumulators d = 2..9 are added into two
 //   64-bit integers per output, again without rounding.
-// The pairs with p + q > 9 are left out: together they are below 2^-8 of the
-// rounding of the operands to 55 bits.  Nothing else is rounded until the
-// final conversion, so the products are at least as accurate as FP64
-// multiply-add chains, and deterministic.
+// The pairs with p + q > 9 are left out: together they are below 2^-59 max|x| max|y|
+// a term.  The sums of a K range are rounded to FP64 once, and so is the result.
+// The order is fixed: equal calls give equal bits.
+//
+// Accuracy.  A real product of rows a and b is off by at most
+//   2^-54 (max|a| sum|b| + sum|a| max|b|) + 2^-59 K max|a| max|b|,
+// where FP64 multiply-adds are off by at most (K + 1) 2^-53 sum|a||b|: at or below
+// them relative to max|a| max|b| (measured 0.1 times their error on rows of even
+// size), and above them relative to sum|a||b| as far as the entries that meet are
+// below the largest.  max and sum are over
+//   an overlap: g, within one K range, for rows a = X_i and b = Y_j.  Rows that
+//     decay in opposite directions over the basis are fine (2^-58 sum|a||b|), rows that
+//     do so within a range are not (decay 1e-13 and back every 128 g: 7e-7);
+//   a rotation: the bands i, for a = X_i(g) / s_i and b = s_i W(i, j), s_i the power of
+//     two of band i's largest entry (k_oz_band_exp): off by 2^-54 of the output
+//     band's terms at their largest, whatever the norms of the bands.
+// The multiply-add forms keep to sum|a||b| and are what a call without the larger
+// workspace runs.  Falling back to them where sum|a||b| is small was not done: bands
+// of a supercell that fold from different k have disjoint entries, and would all.
 //
 // Rows with a NaN or an infinity are marked by their scale and their outputs
 // computed by plain FP64 multiply-adds.
 //
 // Measured (us, 352 x 176 over 37073, one k; FP64 multiply-adds before): overlap
-// 25690 -> 814, rotation 16805 -> 741.  The GEMMs take 574 and 562 of these, a
-// chunk of 128 K (34 pairs: 4.6 us at the tensor cores' peak) in 7.7 us: its
-// pipe is the bound, 60% busy; the slicing kernels run at 4.5 TB/s.
+// 25690 -> 812, rotation 16805 -> 787.  The GEMMs take 575 and 563 of these, a
+// chunk of 128 K (34 pairs: 4.6 us at the tensor cores' peak) in 7.7 us: the copies
+// of 14 digit tiles for 34 products bind (tensor pipe 45% active in captures of one
+// panel); the slicing kernels run at 4.5 TB/s.
 //
 // Kernels (for each complex product as real ones: rows Re and Im stacked, or
 // folded along K where only the real part is kept):
