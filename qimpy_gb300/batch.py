@@ -186,8 +186,8 @@ class Instance:
         # Complex64 subspace products on the CUDA cores: the tensor-core ones take
         # ~0.2 GB of bf16 operand workspace per call on the largest cells, and with
         # many requests' worker threads each caching its own, served runs exhausted
-        # device memory (library handle creation then failed).  (The FP64 ones, at
-        # most some 128 MB of digits and sums, are in EigenServer.estimate_bytes.)
+        # device memory (library handle creation then failed).  (The FP64 ones, up
+        # to 256 MB of digits and sums, are in EigenServer.estimate_bytes.)
         basis.tc_subspace = False
         pad = torch.arange(basis.n_tot)[None, :] < torch.from_numpy(basis.n)[:, None]
         basis.mask = pad.to(self.sphere.device)
@@ -328,9 +328,9 @@ class BatchedHamiltonian:
     plane_chunk_bytes: int = 0
     #: Instances with at least this many (k, band, slab) work units fill the GPU
     #: by themselves (two waves of 152 SMs x 4 CTAs); they run through the
-    #: single-instance call (kernel parameters in constant memory, the
-    #: asynchronous x-pass without per-unit context staging) inside the same
-    #: graph, and only the smaller ones share batched launches.  0 batches all.
+    #: single-instance call (kernel parameters in constant memory, an x-pass on
+    #: tiles of columns without per-unit context staging) inside the same graph,
+    #: and only the smaller ones share batched launches.  0 batches all.
     solo_units: int = 2 * 152 * 4
 
     def __post_init__(self):

@@ -655,9 +655,11 @@ __device__ __forceinline__ void xpair_step(int R, float2* base, const float* V, 
       xpair_last_R<RR>(base, xs, l, L1, lim);                  \
     break;
   switch (R) {
-    QGB_XP(1) QGB_XP(2) QGB_XP(3) QGB_XP(4) QGB_XP(5) QGB_XP(6) QGB_XP(7) QGB_XP(8) QGB_XP(9) QGB_XP(10) QGB_XP(12)
+    QGB_XP(2) QGB_XP(3) QGB_XP(4) QGB_XP(5) QGB_XP(6) QGB_XP(7) QGB_XP(8) QGB_XP(9) QGB_XP(10) QGB_XP(12)
     QGB_XP(14) QGB_XP(15) QGB_XP(16)
-    default: break;
+    default:  // radix 1: the middle step of an axis with L1 = 1
+      if constexpr (STEP == 1) xpair_mid_R<1>(V, l, plane, v_lim, L2, Wx, lim);
+      break;
   }
 #undef QGB_XP
 }

@@ -61,10 +61,10 @@ template <typename L> __device__ __forceinline__ L lane_const(float c) {
 
 template <typename L> struct Lazy {
   L v = 0;
-  float c = 1.0f;        // the value is +-c v; c alone for a literal
-  bool neg = false, scaled = false, literal = false;
+  float c = 1.0f;        // the value is +-c v; a literal is its c alone
+  bool neg = false, scaled = false;
   Lazy() = default;
-  __device__ __forceinline__ explicit Lazy(double x) : c(static_cast<float>(x)), literal(true) {}
+  __device__ __forceinline__ explicit Lazy(double x) : c(static_cast<float>(x)) {}
   __device__ __forceinline__ static Lazy of(L p) {
     Lazy r;
     r.v = p;

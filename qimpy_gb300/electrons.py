@@ -309,7 +309,8 @@ class Electrons:
 
     def hamiltonian(self, C: Wavefunction) -> Wavefunction:
         """HC in one C-ABI call: fused KE + local potential, then the nonlocal
-        term (FP64: ZGEMMs; mixed: tcgen05 split-BF16x3 GEMMs)."""
+        term (FP64: tcgen05 GEMMs of integer slices, multiply-adds where small;
+        mixed: tcgen05 split-BF16x3 GEMMs)."""
         ions = self.ions
         if self.basis.real is not None and self.basis.dtype == torch.complex64:
             HC, projT = ops.hamiltonian_real_mixed(self.basis.real, C.coeff, ions.beta_split, ions.D)
