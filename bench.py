@@ -265,14 +265,12 @@ def roofline_counts(p, b, tables, nb_tile: int, real_bytes: int):
 
 
 # DRAM bytes (read + write) per 32-band si64 block, from ncu captures of the
-# mixed form (`--set full`, default cache control: caches flushed before every
-# kernel, so planes one kernel writes and the next reads count as DRAM traffic
-# although they stay in L2 in a timed run).  Recorded constants of those
-# captures, not measured by this run: the local potential's three kernels as
-# they are now (292.9 MB), the nonlocal chain as captured before its
-# back-projection stored instead of accumulating (195.9 MB; storing skips one
-# 9.5 MB read of HC).
-NCU_DRAM_BYTES_PER_BLOCK = {"local": 292.9e6, "nonlocal": 195.9e6}
+# mixed form (default cache control: caches flushed before every kernel, so planes
+# one kernel writes and the next reads count as DRAM traffic although they stay in
+# L2 in a timed run).  Recorded constants of those captures
+# (profiles/ncu_si64_block.md), not measured by this run: k_ifft_yz, k_xpass and
+# k_fft_yz_gather, and the five kernels of the nonlocal chain in its store form.
+NCU_DRAM_BYTES_PER_BLOCK = {"local": 296.1e6, "nonlocal": 176.6e6}
 
 #: Reference H.psi time over the torch port's (oracle/hpsi_torch.py), si64 by
 #: band count, both on all 8 cores of one x86 host (tests/golden/time_reference_vs_port.py).
@@ -529,9 +527,10 @@ def run_gb300(args, rank, ws, local):
             err = float((Hh.to(dev) - HC).abs().max() / HC.abs().max())
             res["e2e_matches_device_result"] = err
         # our kernels per step: 3 local-potential kernels per FFT block, plus the
-        # nonlocal term once per call: 5 tensor-core chain kernels (mixed) or the
-        # Gram, its reduction, D and the rotation (FP64)
-        res["launches_per_step"] = 3 * len(blocks) + (5 if mixed else 13) * (1 if one_call else len(blocks))
+        # nonlocal term once per call: 5 tensor-core chain kernels (mixed), or slices
+        # and digit GEMMs of 3 panels, their sum, D, the projectors' scales, D proj's
+        # slices, and slices and GEMMs of 2 panels (FP64)
+        res["launches_per_step"] = 3 * len(blocks) + (5 if mixed else 14) * (1 if one_call else len(blocks))
         res["nonlocal_error_word"] = int(ops.device_error_word(dev).item()) if mixed else 0
         res["real_bytes"] = 8 if cdt == torch.complex128 else 4
         res["fft_schedule"] = [list(f) for f in ds.tables.fac]
