@@ -19,8 +19,10 @@
 // its integer pipes 50% and the converting FP64 pipe 39% busy: what is left is
 // latency, at 128 registers a thread and 16 warps an SM.
 //
-// A block with a NaN or an infinity gives NaN (any DFT of it is non-finite in
-// FP64 too).  Values below 2^-960 of an all-tiny block are taken as zero.
+// A block with a NaN or an infinity gives NaN (any DFT of it is non-finite in FP64
+// too), and so does one that holds 2^1018 or more: keeping outputs between that and
+// the largest double took a branch a block, 5% of every FP64 pass.  Numbers are kept
+// to a multiple of 2^-1022.
 #pragma once
 
 #include "codelets.cuh"
@@ -108,10 +110,10 @@ template <int R> constexpr int fx_bits() {
   return 61 - g;
 }
 
-// Largest exponent field of a block of doubles (at least 64, see above).
+// Largest exponent field of a block of doubles, at least `least`.
 template <int R>
-__device__ __forceinline__ int fx_exponent(const double (&re)[R], const double (&im)[R]) {
-  unsigned m = 64u << 20;
+__device__ __forceinline__ int fx_exponent(const double (&re)[R], const double (&im)[R], int least) {
+  unsigned m = static_cast<unsigned>(least) << 20;
 #pragma unroll
   for (int j = 0; j < R; ++j) {
     m = max(m, static_cast<unsigned>(__double2hiint(re[j])) & 0x7FFFFFFFu);
@@ -133,7 +135,7 @@ __device__ __forceinline__ long long fx_from_double(double x, int e) {
   return (static_cast<long long>(m) ^ sg) - sg;
 }
 
-// v 2^k as a double, rounded once (k such that the result is a normal number),
+// v 2^k as a double, rounded once (kLow <= k <= kHigh, see Block),
 // or NaN where `nan` holds its exponent bits.
 __device__ __forceinline__ double fx_to_double(long long v, int k, int nan) {
   const double d = __ll2double_rn(v);
@@ -178,13 +180,14 @@ template <int R> struct Block<float, R> {
 
 template <int R> struct Block<double, R> {
   static constexpr int B = fx_bits<R>();
+  static constexpr int kLow = -1022, kHigh = 962;  // v 2^k of 1 <= |v| < 2^61 is a normal number
   Fx re[R], im[R];
   int k;     // a value is v 2^k
-  bool bad;  // a NaN or an infinity among the inputs
+  bool bad;  // a NaN or an infinity among the inputs, or outputs that could overflow
   __device__ __forceinline__ void load(const double (&x)[R], const double (&y)[R]) {
-    const int e = fx_exponent<R>(x, y);
-    bad = e >= 0x7FF - 8;  // (or so large that an output could overflow)
+    const int e = fx_exponent<R>(x, y, B);  // k >= kLow
     k = e - 1023 - (B - 1);
+    bad = k > kHigh;
 #pragma unroll
     for (int j = 0; j < R; ++j) {
       re[j] = fx_raw(fx_from_double<B>(x[j], e));
@@ -208,14 +211,14 @@ template <int R> struct Block<double, R> {
       mx |= static_cast<unsigned>(a ^ (a >> 31)) | static_cast<unsigned>(b ^ (b >> 31));
     }
     const int e = static_cast<int>(mv >> 20);
-    bad |= e >= 0x7FF - 8;
     const int grown = max(0, 64 - __clz(static_cast<int>(mx)) - B);  // |value| < 2^(B + grown)
     k += e - 1022 + grown;
-    bad |= k + 1023 + B + 8 >= 0x7FF;
-    if (k < -1000) k = -1000;  // products below 2^-940: kept in range
+    bad |= e == 0x7FF || k > kHigh;
+    const int low = max(kLow - k, 0);  // products near the smallest double: as multiples of 2^kLow
+    k += low;
 #pragma unroll
     for (int j = 0; j < R; ++j) {
-      const long long f = fx_from_double<62>(v[j], e + grown);  // |v| 2^(62 - grown), below 2^62
+      const long long f = fx_from_double<62>(v[j], e + grown + low);  // |v| 2^(62 - grown), below 2^62
       int l = static_cast<int>(f);
       if (l == -2147483647 - 1) l = -2147483647;
       const FxConst c{l, static_cast<int>((f - l) >> 32)};
