@@ -42,9 +42,9 @@ struct FxConst {
 };
 __host__ __device__ constexpr FxConst fx_const(double c) {
   const long long v = static_cast<long long>(c * 4611686018427387904.0);
-  int l = static_cast<int>(static_cast<unsigned>(v & 0xFFFFFFFFll));
-  if (l == -2147483647 - 1) l = -2147483647;  // so that it can be negated
-  return FxConst{l, static_cast<int>((v - l) >> 32)};
+  const int l = static_cast<int>(static_cast<unsigned>(v & 0xFFFFFFFFll));
+  // (the low half moves by one unit where it could not be negated, the high half is its own)
+  return FxConst{l == -2147483647 - 1 ? -2147483647 : l, static_cast<int>((v - l) >> 32)};
 }
 
 // A 64-bit integer of a block, |v| < 2^61 where it is multiplied.  Fx(c) is a
@@ -219,8 +219,7 @@ template <int R> struct Block<double, R> {
 #pragma unroll
     for (int j = 0; j < R; ++j) {
       const long long f = fx_from_double<62>(v[j], e + grown + low);  // |v| 2^(62 - grown), below 2^62
-      int l = static_cast<int>(f);
-      if (l == -2147483647 - 1) l = -2147483647;
+      const int l = static_cast<int>(f);
       const FxConst c{l, static_cast<int>((f - l) >> 32)};
       re[j] = fx_mul(re[j], c);
       im[j] = fx_mul(im[j], c);
